@@ -51,6 +51,16 @@ enum SweepMode {
   kDiagBwd = 4,  // z_i = (y_i - sum_upper a z) / a_ii
 };
 
+// A block of at most 32 consecutive rows, one warp's unit of a sweep or
+// factorization.  scan: inside the block a row depends at most on the
+// adjacent one (row - 1 lower, row + 1 upper).
+struct __align__(16) SweepBlock {
+  int id;
+  int base;  // first row
+  int rows;
+  int scan;
+};
+
 // One triangular sweep over a CRS pattern with sorted rows: lo_end[i] is
 // the first entry of row i with column >= i, up_beg[i] the first with
 // column > i (up_beg[i] > lo_end[i] iff the diagonal is stored).
@@ -63,14 +73,14 @@ struct Sweep {
   const void *scale = nullptr;  // SOR modes: per-row multiplier
   int mode = kSorFwd;
   // schedule: blocks in level order, each block's dependency blocks (CSR)
-  const int *order = nullptr;
+  const SweepBlock *order = nullptr;
   const int *dep_off = nullptr;
   const int *dep_ids = nullptr;
 };
 
 // A level schedule of the row blocks for one sweep direction.
 struct Schedule {
-  int *order = nullptr;    // nb block ids, by level
+  SweepBlock *order = nullptr;  // nb blocks, by level
   int *dep_off = nullptr;  // nb + 1
   int *dep_ids = nullptr;  // dependency blocks of each block
   int *level_off = nullptr;  // levels + 1: where each level starts in order
@@ -92,7 +102,9 @@ struct Precond {
   int kind = 0;   // MLSH_PRECOND_SOR / _IC / _ILU
   int dtype = MLSH_F64;
   int n = 0, nnz = 0;
-  unsigned nb = 0;  // row blocks of 32
+  unsigned nb = 0;           // row blocks
+  int *blk_start = nullptr;  // nb + 1: first row of each block
+  int *block_of = nullptr;   // n: each row's block
   Sweep fwd, bwd;
   // owned device buffers
   int *lo_end = nullptr, *up_beg = nullptr;  // A's pattern

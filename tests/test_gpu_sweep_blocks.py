@@ -1,0 +1,75 @@
+"""Row blocks of the sweeps on grids whose lines are not multiples of 32 rows.
+
+Blocks end at 32 rows and, where that shortens the dependency chain, at rows
+that do not depend on their predecessor.  Lines just below, at and above a
+block's 32 rows and twice that, lines of a few rows (where the plain blocks
+stay), and a matrix with no line structure; systems in the single-CTA and in
+the flag-synchronized sweeps.  Factors bit-identical to the sequential
+restatement, applies within the sweeps' bars (1e-12 FP64 / 1e-5 FP32).
+"""
+import numpy as np
+import pytest
+
+from monolish_b200 import _abi
+from monolish_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+SOR, IC, ILU = _abi.PRECOND_SOR, _abi.PRECOND_IC, _abi.PRECOND_ILU
+
+
+def permuted(rp, ci, v, seed):
+    """P A P^T for a random P: no line structure left."""
+    n = len(rp) - 1
+    p = np.random.default_rng(seed).permutation(n)
+    inv = np.argsort(p)
+    rows = []
+    for i in range(n):
+        j = p[i]
+        c, w = inv[ci[rp[j]:rp[j + 1]]], v[rp[j]:rp[j + 1]]
+        o = np.argsort(c)
+        rows.append((c[o], w[o]))
+    return (np.concatenate([[0], np.cumsum([len(c) for c, _ in rows])]).astype(np.int32),
+            np.concatenate([c for c, _ in rows]).astype(np.int32),
+            np.concatenate([w for _, w in rows]))
+
+
+# name: (matrix, most block levels a sweep may have, None: as it comes)
+MATS = {"lines_31": (W.poisson2d(31, 31)[1:], 31),
+        "lines_32": (W.poisson2d(32, 32)[1:], 32),
+        "lines_33": (W.poisson2d(33, 33)[1:], 34),
+        "lines_65": (W.poisson2d(65, 65)[1:], 67),
+        "lines_3": (W.poisson2d(3, 40)[1:], None),
+        "lines_40_of_3": (W.poisson2d(40, 3)[1:], None),
+        "cube_17": (W.poisson3d(17)[1:], 33),
+        "cube_33_flags": (W.poisson3d(33)[1:], 66),
+        "grid_251_flags": (W.poisson2d(251, 251)[1:], 258),
+        "permuted": (permuted(*W.poisson2d(30, 30)[1:], 5), None)}
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("name", sorted(MATS))
+def test_odd_lines(handle, restatement, name, dtype):
+    import torch
+    from monolish_b200 import device as D
+    (rp, ci, v), most = MATS[name]
+    v = v.astype(dtype)
+    n = len(rp) - 1
+    A = D.Crs(handle, n, n, rp, ci, v)
+    r = np.random.default_rng(3).uniform(-1, 1, n).astype(dtype)
+    for kind in (SOR, IC, ILU):
+        pc = D.Precond(A, kind, omega=1.9)
+        lower, upper, blocks = pc.info()
+        assert blocks >= (n + 31) // 32
+        if most is not None:
+            assert max(lower, upper) <= most, (lower, upper)
+        want_f, _ = restatement.precond_factor(rp, ci, v, kind, omega=1.9)
+        assert np.array_equal(pc.factor().cpu().numpy(), want_f)
+        z = torch.zeros(n, dtype=torch.float64 if dtype == np.float64 else torch.float32,
+                        device="cuda")
+        pc.apply(torch.from_numpy(r).cuda(), z)
+        want = restatement.precond_apply(rp, ci, v, kind, r, omega=1.9)
+        err = np.abs(z.cpu().numpy() - want).max() / np.abs(want).max()
+        assert err < (1e-12 if dtype == np.float64 else 1e-5), (kind, err)
+        pc.close()
+    A.close()
