@@ -76,6 +76,10 @@ int mixed_bicgstab_kernels(Handle &h, CsrPlan &p, CsrPlan &p32, double *r64,
                            const mlsh_solver_opts *opts, double inner_tol,
                            mlsh_solver_result *res);
 
+// The handle's work buffer, at least `bytes` long (mlsh_krylov.cu); growing it
+// drops the solver graphs that use the old one.
+int ensure_ws(Handle &h, size_t bytes);
+
 // Solver-side resources kept on the handle / plan (mlsh_krylov.cu).
 void release_solver_graphs(Handle &h);
 void release_plan_extras(CsrPlan &p);

@@ -1215,6 +1215,8 @@ void purge_graphs(Handle &h, const CsrPlan *plan, const void *ws) {
   }
 }
 
+}  // namespace
+
 int ensure_ws(Handle &h, size_t bytes) {
   if (h.ws_bytes >= bytes) return MLSH_SUCCESS;
   if (h.ws) {
@@ -1231,6 +1233,8 @@ int ensure_ws(Handle &h, size_t bytes) {
   h.ws_bytes = bytes;
   return MLSH_SUCCESS;
 }
+
+namespace {
 
 // One system on the cluster engine.  Returns MLSH_NOT_IMPL when the system
 // does not fit it (the caller then uses the kernel engine).

@@ -10,9 +10,13 @@
 //   blas::matvec_T     src/blas/matrix/matvec/crs_matvec.hpp:88-98
 //                      (y_j = sum over rows i in increasing order of a_ij x_i)
 //
-// Design: everything is a stable least-significant-digit radix sort of
-// (32-bit key, 32-bit entry index) pairs, 8 bits per pass, plus binary
-// searches.  Stability makes the results deterministic: a COO sorted by
+// Design: entries are grouped by row (transpose: by column) with a counting
+// pass, a scan and a scatter, and each group is ordered on its own
+// (mlsh_rowsort.cuh).  Matrices with a row of more than kLongCap entries, or
+// with far more rows than entries, take the general form: a stable least-
+// significant-digit radix sort of (32-bit key, 32-bit entry index) pairs, 8
+// bits per pass, plus binary searches.  Both give one and the same order.
+// Stability makes the results deterministic: a COO sorted by
 // column and then by row comes out in (row, col, input position) order, and
 // a CRS re-sorted by column keeps the rows of each column in increasing
 // order -- the order in which the reference's serial loop accumulates
@@ -27,10 +31,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 #include <new>
 #include <vector>
 
 #include "mlsh_core.cuh"
+#include "mlsh_rowsort.cuh"
 
 namespace mlsh {
 
@@ -227,6 +233,100 @@ __global__ void lower_bounds(const unsigned *keys, long long n, int n_out, int *
   }
 }
 
+// ------------------------------------------------- grouping by counting --
+// Items each thread takes at a stride of the block, so that several loads
+// and atomics are in flight.
+constexpr int kGroupItems = 4;
+
+// Entries per key (and the range check of both indices; `other` may be null).
+__global__ void __launch_bounds__(256) count_keys(const int *key, const int *other, long long n,
+                                                  int n_keys, int n_other, unsigned *cnt,
+                                                  SortFlags *flags) {
+  const long long base = (long long)blockIdx.x * (256 * kGroupItems) + threadIdx.x;
+  int k[kGroupItems], o[kGroupItems];
+#pragma unroll
+  for (int u = 0; u < kGroupItems; ++u) {
+    const long long i = base + u * 256;
+    k[u] = i < n ? key[i] : 0;
+    o[u] = i < n && other ? other[i] : 0;
+  }
+#pragma unroll
+  for (int u = 0; u < kGroupItems; ++u) {
+    if (base + u * 256 >= n) break;
+    if (k[u] < 0 || k[u] >= n_keys || (other && (o[u] < 0 || o[u] >= n_other)))
+      flags->bad = 1;
+    else
+      atomicAdd(cnt + k[u], 1u);
+  }
+}
+
+// The largest count.
+__global__ void __launch_bounds__(256) longest_group(const unsigned *cnt, int n_keys,
+                                                     SortFlags *flags) {
+  unsigned m = 0;
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n_keys; i += gridDim.x * 256ll)
+    m = max(m, cnt[i]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(&flags->longest, m);
+}
+
+// Places the COO entries' records through their row's cursor; afterwards
+// cursor[row] is the end of the row's records.
+template <typename T>
+__global__ void __launch_bounds__(256) scatter_coo(const int *row, const int *col, const T *val,
+                                                   long long n, unsigned *cursor,
+                                                   SortRec<T> *rec) {
+  const long long base = (long long)blockIdx.x * (256 * kGroupItems) + threadIdx.x;
+  int r[kGroupItems];
+  SortRec<T> x[kGroupItems];
+#pragma unroll
+  for (int u = 0; u < kGroupItems; ++u) {
+    const long long i = base + u * 256;
+    if (i < n) {
+      r[u] = row[i];
+      x[u] = SortRec<T>{col[i], (unsigned)i, val[i]};
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kGroupItems; ++u)
+    if (base + u * 256 < n) rec[atomicAdd(cursor + r[u], 1u)] = x[u];
+}
+
+// The last row starting at or before entry e, searched in [lo, hi).
+__device__ __forceinline__ int row_of_entry(const int *rp, int lo, int hi, int e) {
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(rp + mid) <= e) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// The same for the entries of a CRS, grouped by column: the rows of a
+// block's entries lie between those of its first and last one.
+template <typename T>
+__global__ void __launch_bounds__(256) scatter_csr(const int *rp, int n_rows, const int *ci,
+                                                   const T *val, long long nnz,
+                                                   unsigned *cursor, SortRec<T> *rec) {
+  __shared__ int s_row[2];
+  const long long b = (long long)blockIdx.x * (256 * kGroupItems);
+  if (threadIdx.x < 2) {
+    const long long e = threadIdx.x == 0 ? b : min(b + 256 * kGroupItems, nnz) - 1;
+    s_row[threadIdx.x] = row_of_entry(rp, 0, n_rows, (int)e);
+  }
+  __syncthreads();
+  const int lo = s_row[0], hi = s_row[1] + 1;
+#pragma unroll
+  for (int u = 0; u < kGroupItems; ++u) {
+    const long long e = b + u * 256 + threadIdx.x;
+    if (e < nnz) {
+      const int c = ci[e];
+      const SortRec<T> x{row_of_entry(rp, lo, hi, (int)e), (unsigned)e, val[e]};
+      rec[atomicAdd(cursor + c, 1u)] = x;
+    }
+  }
+}
+
 // err |= 1 for an index outside [0, n_rows) x [0, n_cols).
 __global__ void coo_range_check(const int *row, const int *col, long long n, int n_rows,
                                 int n_cols, int *err) {
@@ -236,11 +336,14 @@ __global__ void coo_range_check(const int *row, const int *col, long long n, int
       atomicOr(err, 1);
 }
 
-// err |= 2 where rows decrease (the COO -> CRS conversion needs row order).
-__global__ void rows_sorted_check(const int *row, long long n, int *err) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i + 1 < n;
-       i += (long long)gridDim.x * blockDim.x)
-    if (row[i] > row[i + 1]) atomicOr(err, 2);
+// err |= 2 where rows leave [0, n_rows) or decrease (the COO -> CRS conversion
+// needs row order).
+__global__ void rows_sorted_check(const int *row, long long n, int n_rows, int *err) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int r = row[i];
+    if (r < 0 || r >= n_rows || (i + 1 < n && r > row[i + 1])) atomicOr(err, 2);
+  }
 }
 
 // Sorted entries into scratch: rows from the sorted keys, columns and
@@ -390,6 +493,189 @@ int radix_sort_pairs(SortScratch &w, int src, long long n, int bits) {
   return src;
 }
 
+// -------------------------------------------------- grouping: host side --
+// Device scratch of one grouping job of n entries over n_keys groups: kept
+// with the handle up to kKeepScratch (allocating and mapping it anew costs
+// more than sorting: 20 ms for the 16 M-entry case), else the job's own.
+constexpr size_t kKeepScratch = (size_t)1 << 30;
+
+struct GroupScratch {
+  SortFlags *flags = nullptr;
+  unsigned *ends = nullptr;    // n_keys: cursors, then group ends
+  unsigned *kept = nullptr;    // n_keys: kept entries, then output starts
+  unsigned *sums = nullptr;
+  unsigned *long_ids = nullptr;
+  void *rec = nullptr;
+  void *own = nullptr;
+  cudaStream_t s = nullptr;
+
+  int alloc(Handle &h, long long n, long long n_keys) {
+    s = h.stream;
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t keys_b = up(sizeof(unsigned) * (size_t)n_keys);
+    const size_t sums_b = up(sizeof(unsigned) * (size_t)(sort_tiles(n_keys) + 1));
+    const size_t long_b = up(sizeof(unsigned) * (size_t)(n / kSegCap + 1));
+    const size_t total = 256 + 2 * keys_b + sums_b + long_b + 16 * (size_t)n;
+    char *p = nullptr;
+    if (total <= kKeepScratch) {
+      const int st = ensure_ws(h, total);
+      if (st != MLSH_SUCCESS) return st;
+      p = static_cast<char *>(h.ws);
+    } else {
+      if (pool_alloc(&own, total, s) != cudaSuccess) {
+        cudaGetLastError();
+        own = nullptr;
+        return MLSH_ERR_OOM;
+      }
+      p = static_cast<char *>(own);
+    }
+    flags = reinterpret_cast<SortFlags *>(p);
+    ends = reinterpret_cast<unsigned *>(p + 256);
+    kept = reinterpret_cast<unsigned *>(p + 256 + keys_b);
+    sums = reinterpret_cast<unsigned *>(p + 256 + 2 * keys_b);
+    long_ids = reinterpret_cast<unsigned *>(p + 256 + 2 * keys_b + sums_b);
+    rec = p + 256 + 2 * keys_b + sums_b + long_b;
+    return MLSH_SUCCESS;
+  }
+  ~GroupScratch() {
+    if (own) {
+      cudaStreamSynchronize(s);
+      pool_free(own, s);
+    }
+  }
+};
+
+// Keys far more numerous than entries: counting and scanning them would cost
+// more than sorting the entries.
+bool groups_worth(long long n, long long n_keys) { return n_keys <= 4 * n + 4096; }
+
+int read_flags(const GroupScratch &w, Handle &h, SortFlags *out) {
+  static_assert(sizeof(SortFlags) <= 2 * sizeof(double), "host mirror: host_scalars[4..5]");
+  MLSH_CUDA_TRY(cudaMemcpyAsync(&h.host_scalars[4], w.flags, sizeof(SortFlags),
+                                cudaMemcpyDeviceToHost, w.s));
+  MLSH_CUDA_TRY(cudaStreamSynchronize(w.s));
+  std::memcpy(out, &h.host_scalars[4], sizeof(SortFlags));
+  return MLSH_SUCCESS;
+}
+
+unsigned group_blocks(long long n) {
+  return (unsigned)((n + 256 * kGroupItems - 1) / (256 * kGroupItems));
+}
+
+// Counts per key into w.ends; the flags hold the range check and the
+// longest group afterwards.
+int count_groups(GroupScratch &w, Handle &h, const int *key, const int *other, long long n,
+                 int n_keys, int n_other, SortFlags *out) {
+  MLSH_CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(SortFlags), w.s));
+  MLSH_CUDA_TRY(cudaMemsetAsync(w.ends, 0, sizeof(unsigned) * (size_t)n_keys, w.s));
+  count_keys<<<group_blocks(n), 256, 0, w.s>>>(key, other, n, n_keys, n_other, w.ends, w.flags);
+  longest_group<<<grid_for(n_keys), 256, 0, w.s>>>(w.ends, n_keys, w.flags);
+  MLSH_CUDA_TRY(cudaGetLastError());
+  return read_flags(w, h, out);
+}
+
+template <typename T, bool MERGE, bool WRITE>
+int launch_order(const GroupArgs<T> &a, unsigned longest, int num_sms, cudaStream_t s) {
+  const long long per = 32 * kSegWarps;
+  order_groups<T, MERGE, WRITE><<<(unsigned)((a.n_keys + per - 1) / per), kSegWarps * 32, 0, s>>>(
+      a);
+  if (longest > (unsigned)kSegCap) {
+    constexpr auto k = order_long_groups<T, MERGE, WRITE>;
+    MLSH_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongSmem));
+    k<<<(unsigned)num_sms, kLongThreads, kLongSmem, s>>>(a);
+  }
+  MLSH_CUDA_TRY(cudaGetLastError());
+  return MLSH_SUCCESS;
+}
+
+// Orders every group of the scattered records into `out`; with merge only
+// the last entry of each (key, other) stays and *total is what is left.
+template <typename T>
+int order_all(GroupScratch &w, Handle &h, long long n, int n_keys, unsigned longest, bool merge,
+              const SortOut<T> &out, long long *total) {
+  GroupArgs<T> a{};
+  a.rec = static_cast<const SortRec<T> *>(w.rec);
+  a.ends = w.ends;
+  a.n_keys = n_keys;
+  a.long_ids = w.long_ids;
+  a.flags = w.flags;
+  a.collect = 1;
+  a.out = out;
+  *total = n;
+  if (!merge) return launch_order<T, false, true>(a, longest, h.num_sms, w.s);
+  a.kept = w.kept;
+  int st = launch_order<T, true, false>(a, longest, h.num_sms, w.s);
+  if (st != MLSH_SUCCESS) return st;
+  // the last key's count and its exclusive prefix give the total
+  unsigned *host = reinterpret_cast<unsigned *>(&h.host_scalars[4]);
+  MLSH_CUDA_TRY(cudaMemcpyAsync(host, w.kept + n_keys - 1, sizeof(unsigned),
+                                cudaMemcpyDeviceToHost, w.s));
+  scan_exclusive(w.kept, w.kept, n_keys, w.sums, w.s);
+  MLSH_CUDA_TRY(cudaMemcpyAsync(host + 1, w.kept + n_keys - 1, sizeof(unsigned),
+                                cudaMemcpyDeviceToHost, w.s));
+  a.starts = w.kept;
+  a.kept = nullptr;
+  a.collect = 0;
+  st = launch_order<T, true, true>(a, longest, h.num_sms, w.s);
+  if (st != MLSH_SUCCESS) return st;
+  MLSH_CUDA_TRY(cudaStreamSynchronize(w.s));
+  *total = (long long)host[0] + host[1];
+  return MLSH_SUCCESS;
+}
+
+// COO sort by grouping; *done = false when the general sort has to take it
+// (nothing has been written then).
+template <typename T>
+int coo_group_sort(Handle &h, int n_rows, int n_cols, long long n, int *row, int *col, T *val,
+                   bool merge, long long *total, bool *done) {
+  *done = false;
+  GroupScratch w;
+  int st = w.alloc(h, n, n_rows);
+  if (st != MLSH_SUCCESS) return st;
+  SortFlags f;
+  st = count_groups(w, h, row, col, n, n_rows, n_cols, &f);
+  if (st != MLSH_SUCCESS) return st;
+  if (f.bad) return MLSH_ERR_INVALID_ARG;
+  if (f.longest > (unsigned)kLongCap) return MLSH_SUCCESS;
+  *done = true;
+  scan_exclusive(w.ends, w.ends, n_rows, w.sums, w.s);
+  scatter_coo<T><<<group_blocks(n), 256, 0, w.s>>>(row, col, val, n, w.ends,
+                                                   static_cast<SortRec<T> *>(w.rec));
+  return order_all<T>(w, h, n, n_rows, f.longest, merge, SortOut<T>{row, col, val, nullptr},
+                      total);
+}
+
+// The transpose by grouping, as coo_group_sort.
+template <typename T>
+int transpose_group(Handle &h, int n_rows, int n_cols, long long nnz, const int *rp,
+                    const int *ci, const T *val, int *rp_t, int *ci_t, T *val_t,
+                    unsigned *perm_out, bool *done) {
+  *done = false;
+  GroupScratch w;
+  int st = w.alloc(h, nnz, n_cols);
+  if (st != MLSH_SUCCESS) return st;
+  SortFlags f;
+  st = count_groups(w, h, ci, nullptr, nnz, n_cols, 0, &f);
+  if (st != MLSH_SUCCESS) return st;
+  if (f.bad) return MLSH_ERR_INVALID_CSR;
+  if (f.longest > (unsigned)kLongCap) return MLSH_SUCCESS;
+  *done = true;
+  scan_exclusive(w.ends, w.ends, n_cols, w.sums, w.s);
+  MLSH_CUDA_TRY(cudaMemcpyAsync(rp_t, w.ends, sizeof(int) * (size_t)n_cols,
+                                cudaMemcpyDeviceToDevice, w.s));
+  scatter_csr<T><<<group_blocks(nnz), 256, 0, w.s>>>(rp, n_rows, ci, val, nnz, w.ends,
+                                                     static_cast<SortRec<T> *>(w.rec));
+  // the last column's end is the entry count
+  MLSH_CUDA_TRY(cudaMemcpyAsync(rp_t + n_cols, w.ends + n_cols - 1, sizeof(int),
+                                cudaMemcpyDeviceToDevice, w.s));
+  long long total = 0;
+  st = order_all<T>(w, h, nnz, n_cols, f.longest, false,
+                    SortOut<T>{nullptr, ci_t, val_t, perm_out}, &total);
+  if (st != MLSH_SUCCESS) return st;
+  MLSH_CUDA_TRY(cudaStreamSynchronize(w.s));
+  return MLSH_SUCCESS;
+}
+
 // Reads back the device error word (synchronizes the stream).
 int read_flag(const int *d_flag, cudaStream_t s, int *out) {
   MLSH_CUDA_TRY(cudaMemcpyAsync(out, d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -431,8 +717,20 @@ int transpose_build(Handle &h, int n_rows, int n_cols, int nnz, const int *rp, c
     MLSH_CUDA_TRY(cudaStreamSynchronize(s));
     return MLSH_SUCCESS;
   }
+  int st = MLSH_SUCCESS;
+  if (groups_worth(nnz, n_cols)) {
+    bool done = false;
+    st = dtype == MLSH_F64
+             ? transpose_group<double>(h, n_rows, n_cols, nnz, rp, ci,
+                                       static_cast<const double *>(val), rp_t, ci_t,
+                                       static_cast<double *>(val_t), perm_out, &done)
+             : transpose_group<float>(h, n_rows, n_cols, nnz, rp, ci,
+                                      static_cast<const float *>(val), rp_t, ci_t,
+                                      static_cast<float *>(val_t), perm_out, &done);
+    if (st != MLSH_SUCCESS || done) return st;
+  }
   SortScratch w;
-  int st = w.alloc(nnz, 256, s);
+  st = w.alloc(nnz, 256, s);
   if (st != MLSH_SUCCESS) return st;
   int *d_err = reinterpret_cast<int *>(w.extra);
   MLSH_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s));
@@ -571,9 +869,28 @@ int mlsh_coo_sort(mlsh_handle hs, int n_rows, int n_cols, int64_t nnz, int *d_ro
   const size_t esz = (size_t)dtype_size(dtype);
   const size_t vec4 = ((size_t)n * 4 + 255) / 256 * 256;
   const size_t vecv = ((size_t)n * esz + 255) / 256 * 256;
+  // By counting where no row is longer than the ordering kernels take and the
+  // rows are not far more than the entries; the radix sort otherwise.  Sort,
+  // merge and row pointers of 16.1 M shuffled triplets of the 128^3 7-point
+  // matrix (FP64): 1.52 ms, by the radix sort 13.1 ms; the transpose of the
+  // 1,000,003-row Zipf(2) matrix with its first product 7.4 against 14.6 ms.
+  int st = MLSH_SUCCESS;
+  if (groups_worth(n, n_rows)) {
+    bool done = false;
+    long long left = 0;
+    st = esz == 8 ? coo_group_sort<double>(h, n_rows, n_cols, n, d_row, d_col,
+                                           static_cast<double *>(d_val), merge != 0, &left, &done)
+                  : coo_group_sort<float>(h, n_rows, n_cols, n, d_row, d_col,
+                                          static_cast<float *>(d_val), merge != 0, &left, &done);
+    if (st == MLSH_SUCCESS && done) {
+      MLSH_CUDA_TRY(cudaStreamSynchronize(s));
+      *new_nnz = left;
+    }
+    if (st != MLSH_SUCCESS || done) return st;
+  }
   // extra: error word, sorted rows/cols/values, run flags and positions
   SortScratch w;
-  int st = w.alloc(n, 256 + 4 * vec4 + vecv, s);
+  st = w.alloc(n, 256 + 4 * vec4 + vecv, s);
   if (st != MLSH_SUCCESS) return st;
   int *d_err = reinterpret_cast<int *>(w.extra);
   int *t_row = reinterpret_cast<int *>(w.extra + 256);
@@ -631,26 +948,21 @@ int mlsh_coo_to_csr(mlsh_handle hs, int n_rows, int64_t nnz, const int *d_row, i
   if (!hs || n_rows < 0 || nnz < 0 || nnz > INT32_MAX || !d_row_ptr || (nnz > 0 && !d_row))
     return MLSH_ERR_INVALID_ARG;
   cudaStream_t s = hs->h.stream;
-  if (nnz > 0) {
-    int *d_err = nullptr;
-    if (pool_alloc(&d_err, sizeof(int), s) != cudaSuccess) {
-      cudaGetLastError();
-      return MLSH_ERR_OOM;
-    }
-    cudaMemsetAsync(d_err, 0, sizeof(int), s);
-    coo_range_check<<<grid_for(nnz), 256, 0, s>>>(d_row, nullptr, nnz, n_rows, 0, d_err);
-    rows_sorted_check<<<grid_for(nnz), 256, 0, s>>>(d_row, nnz, d_err);
-    int err = 0;
-    const int st = read_flag(d_err, s, &err);
-    pool_free(d_err, s);
-    if (st != MLSH_SUCCESS) return st;
-    if (err) return MLSH_ERR_INVALID_CSR;
-  }
+  // the check's word and its host mirror live with the handle; the searches
+  // stay in bounds whatever the rows hold, so one wait covers both launches
+  Handle &h = hs->h;
+  int *d_err = reinterpret_cast<int *>(h.scalars + 6);
+  MLSH_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s));
+  if (nnz > 0) rows_sorted_check<<<grid_for(nnz), 256, 0, s>>>(d_row, nnz, n_rows, d_err);
   lower_bounds<<<grid_for((long long)n_rows + 1), 256, 0, s>>>(
       reinterpret_cast<const unsigned *>(d_row), nnz, n_rows, d_row_ptr);
   MLSH_CUDA_TRY(cudaGetLastError());
+  MLSH_CUDA_TRY(cudaMemcpyAsync(&h.host_scalars[6], d_err, sizeof(int), cudaMemcpyDeviceToHost,
+                                s));
   MLSH_CUDA_TRY(cudaStreamSynchronize(s));
-  return MLSH_SUCCESS;
+  int err = 0;
+  std::memcpy(&err, &h.host_scalars[6], sizeof(int));
+  return err ? MLSH_ERR_INVALID_CSR : MLSH_SUCCESS;
 }
 
 int mlsh_csr_transpose(mlsh_handle hs, int n_rows, int n_cols, int nnz, const int *d_rp,
