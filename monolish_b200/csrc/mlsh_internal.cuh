@@ -117,7 +117,9 @@ struct Handle {
   double *scalars = nullptr;     // 8 doubles of device results
   SolverState *state = nullptr;
   SolverState *host_state = nullptr;  // pinned mirror
-  double *host_scalars = nullptr;     // pinned
+  double *host_scalars = nullptr;     // pinned, 8 doubles; [2]: a dot's result
+                                      // and [3]: its number, written by kernels
+  unsigned long long dots = 0;        // host-waited reductions so far
   int *err_flag = nullptr;            // device: nonzero after a timeout
   cudaStream_t capture_stream = nullptr;  // private stream for graph capture
   void *ws = nullptr;                 // solver work vectors

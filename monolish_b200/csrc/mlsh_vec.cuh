@@ -131,6 +131,39 @@ struct Nrm2Body : NoPrep {
   __device__ void finish(const double *s) { *out = sqrt(s[0]); }
 };
 
+// The same sums for a caller that waits: the result goes straight to mapped
+// host memory, then the call's number, which the host watches.
+struct HostResult {
+  double *value;
+  unsigned long long *ready;
+  unsigned long long number;
+  __device__ void publish(double v) const {
+    *(volatile double *)value = v;
+    __threadfence_system();
+    *(volatile unsigned long long *)ready = number;
+  }
+};
+template <typename T>
+struct DotHostBody : NoPrep {
+  const T *x;
+  const T *y;
+  HostResult out;
+  __device__ void operator()(int64_t i, double *acc) const {
+    acc[0] += (double)x[i] * (double)y[i];
+  }
+  __device__ void finish(const double *s) { out.publish(s[0]); }
+};
+template <typename T>
+struct Nrm2HostBody : NoPrep {
+  const T *x;
+  HostResult out;
+  __device__ void operator()(int64_t i, double *acc) const {
+    const double v = (double)x[i];
+    acc[0] += v * v;
+  }
+  __device__ void finish(const double *s) { out.publish(sqrt(s[0])); }
+};
+
 template <typename T>
 struct AxpyBody : NoPrep {  // y = alpha*x + y
   T alpha;
