@@ -412,8 +412,10 @@ int mlsh_precond_destroy(mlsh_precond pc);
  * (levels_lower + levels_upper) such hops -- and the block count. */
 int mlsh_precond_info(mlsh_precond pc, int *levels_lower, int *levels_upper,
                       int64_t *blocks);
-/* Which kernel runs each sweep: MLSH_SWEEP_FLAGS (blocks spread over the
- * GPU, one warp per block, per-block flags between warps), MLSH_SWEEP_CTA
+/* Which kernel runs each sweep: MLSH_SWEEP_FLAGS (blocks spread over several
+ * CTAs: over the GPU with per-block flags between warps, or, for stencil
+ * matrices whose solution fits a cluster's shared memory, over one cluster
+ * whose CTAs meet between levels), MLSH_SWEEP_CTA
  * (one CTA, the solution in shared memory, a barrier between levels) or
  * MLSH_SWEEP_RING (one CTA as before, each block's matrix-only row state
  * precomputed at creation and streamed into a shared-memory ring by bulk

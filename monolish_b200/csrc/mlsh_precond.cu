@@ -25,6 +25,7 @@
 #include "mlsh_core.cuh"
 #include "mlsh_precond.cuh"
 #include "mlsh_ptx.cuh"
+#include "mlsh_sweep_cluster.cuh"
 
 namespace mlsh {
 namespace {
@@ -1025,6 +1026,48 @@ int configure_cta() {
   return MLSH_SUCCESS;
 }
 
+template <typename T, int MODE>
+size_t cluster_sweep_smem(unsigned nb, int levels, int ctas) {
+  const size_t most = ((size_t)nb + ctas - 1) / ctas;
+  return most * 32 * sizeof(T) + sizeof(int) * ((size_t)levels + 1);
+}
+
+template <typename T, int MODE>
+cudaError_t cluster_sweep_config(unsigned nb, int levels, int ctas, cudaStream_t s,
+                                 cudaLaunchConfig_t *cfg, cudaLaunchAttribute *at) {
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3((unsigned)ctas);
+  cfg->blockDim = dim3(kClSweepThreads);
+  cfg->dynamicSmemBytes = cluster_sweep_smem<T, MODE>(nb, levels, ctas);
+  cfg->stream = s;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)ctas;
+  at->val.clusterDim.y = 1;
+  at->val.clusterDim.z = 1;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+  return cudaSuccess;
+}
+
+template <typename T, int MODE>
+cudaError_t cluster_sweep_launch(const SweepArgs<T> &a, const Schedule &sc, cudaStream_t s) {
+  ClusterSweepArgs<T> c;
+  c.order = a.order;
+  c.rec = static_cast<const unsigned char *>(sc.cluster_rec);
+  c.level_off = sc.level_off;
+  c.levels = sc.levels;
+  c.nb = (int)a.nb;
+  c.rhs = a.rhs;
+  c.out = a.out;
+  c.done = a.done;
+  c.err = a.err;
+  c.polls = a.polls;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  cluster_sweep_config<T, MODE>(a.nb, sc.levels, sc.ctas, s, &cfg, &at);
+  return cudaLaunchKernelEx(&cfg, sweep_cluster_kernel<T, MODE>, c);
+}
+
 template <typename T>
 cudaError_t sweep_launch_t(const Precond &pc, const Sweep &sw, bool backward, const void *rhs,
                            void *out, const int *done, int *err, cudaStream_t s) {
@@ -1048,6 +1091,15 @@ cudaError_t sweep_launch_t(const Precond &pc, const Sweep &sw, bool backward, co
   a.dep_ids = sw.dep_ids;
   a.polls = pc.wait_polls;
   const Schedule &sc = backward ? pc.sbwd : pc.sfwd;
+  if (sc.ctas > 0) {
+    switch (sw.mode) {
+      case kSorFwd: return cluster_sweep_launch<T, kSorFwd>(a, sc, s);
+      case kUnitFwd: return cluster_sweep_launch<T, kUnitFwd>(a, sc, s);
+      case kDiagFwd: return cluster_sweep_launch<T, kDiagFwd>(a, sc, s);
+      case kSorBwd: return cluster_sweep_launch<T, kSorBwd>(a, sc, s);
+      default: return cluster_sweep_launch<T, kDiagBwd>(a, sc, s);
+    }
+  }
   const size_t xbytes = cta_smem_bytes<T>(pc.n, pc.nb, sc.levels);
   if (xbytes <= kCtaSweepBytes) {
     switch (sw.mode) {
@@ -1134,7 +1186,8 @@ void precond_release(Precond &pc) {
                   pc.scale,         pc.tmp,           pc.ticket,        pc.flags,
                   pc.sfwd.order,    pc.sfwd.dep_off,  pc.sfwd.dep_ids,  pc.sbwd.order,
                   pc.sbwd.dep_off,  pc.sbwd.dep_ids,  pc.sfwd.level_off, pc.sbwd.level_off,
-                  pc.sfwd.rec,      pc.sbwd.rec,      pc.blk_start,     pc.block_of};
+                  pc.sfwd.rec,      pc.sbwd.rec,      pc.blk_start,     pc.block_of,
+                  pc.sfwd.cluster_rec, pc.sbwd.cluster_rec};
   for (void *b : bufs) pool_free(b, s);
   pc.sfwd = Schedule{};
   pc.sbwd = Schedule{};
@@ -1557,15 +1610,91 @@ int build_records_t(Handle &h, const Precond &pc, const Sweep &sw, Schedule &sc)
   return MLSH_SUCCESS;
 }
 
-int build_records(Handle &h, Precond &pc) {
-  int st = MLSH_SUCCESS;
-  if (pc.dtype == MLSH_F64) {
-    st = build_records_t<double>(h, pc, pc.fwd, pc.sfwd);
-    if (st == MLSH_SUCCESS) st = build_records_t<double>(h, pc, pc.bwd, pc.sbwd);
-  } else {
-    st = build_records_t<float>(h, pc, pc.fwd, pc.sfwd);
-    if (st == MLSH_SUCCESS) st = build_records_t<float>(h, pc, pc.bwd, pc.sbwd);
+// order_index[block] = the block's place in the level order.
+__global__ void order_index_kernel(const SweepBlock *order, unsigned nb, int *order_index) {
+  const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < nb) order_index[order[q].id] = (int)q;
+}
+
+// The cluster form of a sweep that would otherwise run over the whole GPU
+// through L2 flags: where a cluster (16 CTAs, else 8) can be resident with the
+// solution in its shared memory, every block is resolved by the scan and no
+// row has more than four entries outside its block.
+template <typename T, int MODE>
+int build_cluster_mode(Handle &h, const Precond &pc, const Sweep &sw, Schedule &sc) {
+  cudaStream_t s = h.stream;
+  auto k = sweep_cluster_kernel<T, MODE>;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSweepSmem) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return MLSH_SUCCESS;
   }
+  int ctas = 0;
+  for (int c = kClSweepMaxCtas; c >= 8 && ctas == 0; c >>= 1) {
+    if (cluster_sweep_smem<T, MODE>(pc.nb, sc.levels, c) > kClSweepSmem) break;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    cluster_sweep_config<T, MODE>(pc.nb, sc.levels, c, nullptr, &cfg, &at);
+    int active = 0;
+    if (cudaOccupancyMaxActiveClusters(&active, (void *)k, &cfg) == cudaSuccess && active > 0)
+      ctas = c;
+    else
+      cudaGetLastError();
+  }
+  if (ctas == 0) return MLSH_SUCCESS;
+  using R = ClusterRec<T, MODE>;
+  int *index = nullptr;  // [nb] and one flag
+  unsigned char *rec = nullptr;
+  MLSH_CUDA_TRY(pool_alloc(&index, sizeof(int) * ((size_t)pc.nb + 1), s));
+  if (pool_alloc(&rec, (size_t)R::kBytes * pc.nb, s) != cudaSuccess) {
+    cudaGetLastError();
+    pool_free(index, s);
+    return MLSH_SUCCESS;  // no room: the flag sweep stays
+  }
+  MLSH_CUDA_TRY(cudaMemsetAsync(index + pc.nb, 0, sizeof(int), s));
+  order_index_kernel<<<grid_of(pc.nb, 256), 256, 0, s>>>(sw.order, pc.nb, index);
+  cluster_rec_kernel<T, MODE><<<grid_of(pc.nb, 8), 256, 0, s>>>(
+      sw, pc.block_of, index, (int)pc.nb, ctas, rec, index + pc.nb);
+  MLSH_CUDA_TRY(cudaGetLastError());
+  int bad = 0;
+  MLSH_CUDA_TRY(cudaMemcpyAsync(&bad, index + pc.nb, sizeof(int), cudaMemcpyDeviceToHost, s));
+  MLSH_CUDA_TRY(cudaStreamSynchronize(s));
+  pool_free(index, s);
+  if (bad) {
+    pool_free(rec, s);
+    return MLSH_SUCCESS;
+  }
+  sc.cluster_rec = rec;
+  sc.ctas = ctas;
+  return MLSH_SUCCESS;
+}
+
+template <typename T>
+int build_cluster_t(Handle &h, const Precond &pc, const Sweep &sw, Schedule &sc) {
+  if (sc.order == nullptr || pc.nb == 0 || sc.levels == 0 ||
+      cta_smem_bytes<T>(pc.n, pc.nb, sc.levels) <= kCtaSweepBytes)
+    return MLSH_SUCCESS;
+  switch (sw.mode) {
+    case kSorFwd: return build_cluster_mode<T, kSorFwd>(h, pc, sw, sc);
+    case kUnitFwd: return build_cluster_mode<T, kUnitFwd>(h, pc, sw, sc);
+    case kDiagFwd: return build_cluster_mode<T, kDiagFwd>(h, pc, sw, sc);
+    case kSorBwd: return build_cluster_mode<T, kSorBwd>(h, pc, sw, sc);
+    default: return build_cluster_mode<T, kDiagBwd>(h, pc, sw, sc);
+  }
+}
+
+template <typename T>
+int build_forms_t(Handle &h, Precond &pc) {
+  int st = build_records_t<T>(h, pc, pc.fwd, pc.sfwd);
+  if (st == MLSH_SUCCESS) st = build_records_t<T>(h, pc, pc.bwd, pc.sbwd);
+  if (st == MLSH_SUCCESS) st = build_cluster_t<T>(h, pc, pc.fwd, pc.sfwd);
+  if (st == MLSH_SUCCESS) st = build_cluster_t<T>(h, pc, pc.bwd, pc.sbwd);
+  return st;
+}
+
+int build_records(Handle &h, Precond &pc) {
+  int st = pc.dtype == MLSH_F64 ? build_forms_t<double>(h, pc) : build_forms_t<float>(h, pc);
   if (st == MLSH_SUCCESS) MLSH_CUDA_TRY(cudaStreamSynchronize(h.stream));
   return st;
 }

@@ -92,6 +92,10 @@ struct Schedule {
   // (0: the sweep does not take the ring form)
   void *rec = nullptr;
   int ring = 0;
+  // cluster sweep (mlsh_sweep_cluster.cuh): its records and its CTAs (0: the
+  // sweep does not take that form)
+  void *cluster_rec = nullptr;
+  int ctas = 0;
 };
 
 constexpr unsigned kDefaultWaitPolls = 1u << 22;  // a few seconds of polling

@@ -3,8 +3,8 @@
 Blocks end at 32 rows and, where that shortens the dependency chain, at rows
 that do not depend on their predecessor.  Lines just below, at and above a
 block's 32 rows and twice that, lines of a few rows (where the plain blocks
-stay), and a matrix with no line structure; systems in the single-CTA and in
-the flag-synchronized sweeps.  Factors bit-identical to the sequential
+stay), and a matrix with no line structure; systems in the single-CTA, the
+cluster and the flag-synchronized sweeps.  Factors bit-identical to the sequential
 restatement, applies within the sweeps' bars (1e-12 FP64 / 1e-5 FP32).
 """
 import numpy as np
@@ -34,6 +34,25 @@ def permuted(rp, ci, v, seed):
             np.concatenate([w for _, w in rows]))
 
 
+def banded(n, offsets, line):
+    """Symmetric, diagonally dominant: entries at +-offsets; the offset 1 stops
+    at the ends of lines."""
+    rng = np.random.default_rng(len(offsets))
+    row, col, val = [np.arange(n)], [np.arange(n)], [np.full(n, 2.0 * len(offsets) + 1)]
+    for o in offsets:
+        i = np.arange(n - o)
+        if o == 1:
+            i = i[(i + 1) % line != 0]
+        w = rng.uniform(-1, 1, len(i))
+        row += [i, i + o]
+        col += [i + o, i]
+        val += [w, w]
+    row, col, val = np.concatenate(row), np.concatenate(col), np.concatenate(val)
+    o = np.lexsort((col, row))
+    rp = np.searchsorted(row[o], np.arange(n + 1)).astype(np.int32)
+    return rp, col[o].astype(np.int32), val[o]
+
+
 # name: (matrix, most block levels a sweep may have, None: as it comes)
 MATS = {"lines_31": (W.poisson2d(31, 31)[1:], 31),
         "lines_32": (W.poisson2d(32, 32)[1:], 32),
@@ -44,6 +63,10 @@ MATS = {"lines_31": (W.poisson2d(31, 31)[1:], 31),
         "cube_17": (W.poisson3d(17)[1:], 33),
         "cube_33_flags": (W.poisson3d(33)[1:], 66),
         "grid_251_flags": (W.poisson2d(251, 251)[1:], 258),
+        # four entries a row below its block (on one cluster), five (not); the
+        # solutions are past a single CTA's shared memory in both precisions
+        "four_outside": (banded(60000, [1, 300, 600, 900, 1200], 300)[:], None),
+        "five_outside": (banded(60000, [1, 300, 600, 900, 1200, 1500], 300)[:], None),
         "permuted": (permuted(*W.poisson2d(30, 30)[1:], 5), None)}
 
 
