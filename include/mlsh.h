@@ -286,7 +286,11 @@ int mlsh_fill(mlsh_handle handle, int dtype, int64_t n, double value,
  *            wall-clock budget of 60 s per solve ends a solve that does not
  *            terminate with MLSH_ERR_TIMEOUT.
  *   AUTO     CLUSTER when the system fits and maxiter <= 2,000,000, else
- *            KERNELS. */
+ *            KERNELS.  CG of 32,769 rows and more, up to 4,096 FP64 or
+ *            8,192 FP32 rows an SM (606,208 / 1,212,416 on 148 SMs; rows of
+ *            up to 16 entries): the same single launch over
+ *            the whole GPU (a cooperative launch with the CLUSTER budget),
+ *            unless a solve server runs in the process. */
 #define MLSH_ENGINE_AUTO 0
 #define MLSH_ENGINE_KERNELS 1
 #define MLSH_ENGINE_CLUSTER 2

@@ -31,6 +31,9 @@ struct BatchGroup {
   int first = 0;  // index of the group's first record in the system array
   int count = 0;
   cudaStream_t stream = nullptr;
+  int slots = 0;         // CG: slots of the launch (0: the row-loop kernel)
+  int n_clusters = 0;
+  size_t space_off = 0;   // its workspace in B.space
 };
 
 struct Batch {
@@ -53,6 +56,10 @@ struct Batch {
   ClusterSystem *h_sys = nullptr;     // pinned mirror
   unsigned *d_queue = nullptr;        // one counter per group
   void *ws = nullptr;                 // inverse diagonal + BiCGSTAB r0
+  int *d_longest = nullptr;           // longest row of each system
+  std::vector<int> longest;
+  void *space = nullptr;              // CG: the groups' matrix slices
+  size_t space_bytes = 0;
   cudaEvent_t done_event = nullptr;
 };
 
@@ -134,7 +141,18 @@ void free_batch(Batch &B) {
   cudaFree(B.d_queue);
   cudaFree(B.ws);
   cudaFree(B.val32);
+  cudaFree(B.d_longest);
+  cudaFree(B.space);
   if (B.done_event) cudaEventDestroy(B.done_event);
+}
+
+// Longest row of system blockIdx.x; row_off[k] is where system k's rows start.
+__global__ void __launch_bounds__(256) longest_rows(const ClusterSystem *sys, int *out) {
+  const int *rp = sys[blockIdx.x].rp;
+  int m = 0;
+  for (int i = threadIdx.x; i < sys[blockIdx.x].n; i += 256) m = max(m, rp[i + 1] - rp[i]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(out + blockIdx.x, m);
 }
 
 __global__ void values_to_f32(const double *v, int64_t n, float *out) {
@@ -189,6 +207,7 @@ int mlsh_batch_create(mlsh_handle hs, int n_systems, const int64_t *row_off,
   bool ok = cudaMalloc(&B.d_sys, sizeof(ClusterSystem) * n_rec) == cudaSuccess &&
             cudaMallocHost(&B.h_sys, sizeof(ClusterSystem) * n_rec) == cudaSuccess &&
             cudaMalloc(&B.d_queue, sizeof(unsigned) * kMaxBatchGroups) == cudaSuccess &&
+            cudaMalloc(&B.d_longest, sizeof(int) * n_rec) == cudaSuccess &&
             cudaMalloc(&B.ws, 2 * esz * (size_t)std::max<int64_t>(B.total_rows, 1) + 256) ==
                 cudaSuccess &&
             cudaEventCreateWithFlags(&B.done_event, cudaEventDisableTiming) == cudaSuccess;
@@ -260,19 +279,51 @@ int batch_run(Handle &h, Batch &B, int kind, const void *d_b, void *d_x, const d
   MLSH_CUDA_TRY(cudaMemcpyAsync(B.d_sys, B.h_sys, sizeof(ClusterSystem) * B.n_systems,
                                 cudaMemcpyHostToDevice, h.stream));
   MLSH_CUDA_TRY(cudaMemsetAsync(B.d_queue, 0, sizeof(unsigned) * kMaxBatchGroups, h.stream));
+  const int n_groups = (int)groups.size();
+  // CG: the longest row of each group decides its kernel and its workspace
+  // (read anew each time: the caller owns the row pointers)
+  if (kind == 0) {
+    MLSH_CUDA_TRY(cudaMemsetAsync(B.d_longest, 0, sizeof(int) * B.n_systems, h.stream));
+    longest_rows<<<(unsigned)B.n_systems, 256, 0, h.stream>>>(B.d_sys, B.d_longest);
+    MLSH_CUDA_TRY(cudaGetLastError());
+    B.longest.resize((size_t)B.n_systems);
+    MLSH_CUDA_TRY(cudaMemcpyAsync(B.longest.data(), B.d_longest, sizeof(int) * B.n_systems,
+                                  cudaMemcpyDeviceToHost, h.stream));
+    MLSH_CUDA_TRY(cudaStreamSynchronize(h.stream));
+  }
+  size_t space = 0;
+  for (BatchGroup &g : groups) {
+    g.slots = 0;
+    if (kind == 0) {
+      int m = 0;
+      for (int i = g.first; i < g.first + g.count; ++i) m = std::max(m, B.longest[(size_t)i]);
+      g.slots = cluster_cg_slots(kind, dt, g.rpc, m);
+    }
+    g.n_clusters = cluster_max_active(kind, dt, jac, g.rpc, g.csize, g.slots);
+    if (g.n_clusters < 1) return MLSH_NOT_IMPL;
+    g.n_clusters = std::min(g.n_clusters, g.count);
+    g.space_off = space;
+    space += (size_t)g.n_clusters * g.csize * cluster_cg_workspace(dt, g.rpc, g.slots);
+  }
+  if (space > B.space_bytes) {
+    cudaFree(B.space);
+    B.space = nullptr;
+    B.space_bytes = 0;
+    if (cudaMalloc(&B.space, space) != cudaSuccess) {
+      cudaGetLastError();
+      return MLSH_ERR_OOM;
+    }
+    B.space_bytes = space;
+  }
   MLSH_CUDA_TRY(cudaEventRecord(B.done_event, h.stream));
   // one stream per group, ordered after the uploads on the handle's stream
-  const int n_groups = (int)groups.size();
   for (int gi = 0; gi < n_groups; ++gi) {
     BatchGroup &g = groups[gi];
     if (!g.stream) MLSH_CUDA_TRY(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
     MLSH_CUDA_TRY(cudaStreamWaitEvent(g.stream, B.done_event, 0));
-    int n_clusters = cluster_max_active(kind, dt, jac, g.rpc, g.csize);
-    if (n_clusters < 1) return MLSH_NOT_IMPL;
-    n_clusters = std::min(n_clusters, g.count);
     const int st = cluster_launch(h, kind, dt, jac, B.d_sys + g.first, g.count, B.d_queue + gi,
-                                  g.rpc, g.csize, n_clusters, cluster_budget(opts), g.stream,
-                                  delta);
+                                  g.rpc, g.csize, g.n_clusters, cluster_budget(opts), g.stream,
+                                  delta, g.slots, static_cast<char *>(B.space) + g.space_off);
     if (st != MLSH_SUCCESS) return st;
   }
   for (int gi = 0; gi < n_groups; ++gi) {

@@ -625,11 +625,14 @@ int cluster_rows_for(int kind, int dtype, int64_t n, int requested) {
 
 int cluster_launch(const Handle &h, int kind, int dtype, bool jac, ClusterSystem *d_systems,
                    int n_systems, unsigned *d_queue, int rpc, int csize, int n_clusters,
-                   double budget_s, cudaStream_t stream, double delta) {
+                   double budget_s, cudaStream_t stream, double delta, int slots, void *space) {
   (void)h;
   if (set_cluster_attributes() != MLSH_SUCCESS) return MLSH_NOT_IMPL;
   int shift = 0;
   while ((1 << shift) < rpc) ++shift;
+  if (slots > 0)
+    return cluster_cg_launch(dtype, jac, d_systems, n_systems, d_queue, rpc, csize, n_clusters,
+                             budget_s, stream, slots, space);
   ClusterArgs a = {};
   a.systems = d_systems;
   a.n_systems = n_systems;
@@ -656,9 +659,10 @@ int cluster_launch(const Handle &h, int kind, int dtype, bool jac, ClusterSystem
   return MLSH_SUCCESS;
 }
 
-int cluster_max_active(int kind, int dtype, bool jac, int rpc, int csize) {
+int cluster_max_active(int kind, int dtype, bool jac, int rpc, int csize, int slots) {
   if (set_cluster_attributes() != MLSH_SUCCESS) return 0;
   cudaLaunchAttribute attr[1];
+  if (slots > 0) return cluster_cg_max_active(dtype, rpc, csize, slots);
   cudaLaunchConfig_t cfg =
       cluster_config(csize, 1, (size_t)cluster_nvec(kind) * rpc * dtype_size(dtype), nullptr,
                      attr);

@@ -43,16 +43,39 @@ struct ClusterSystem;
 // Rows per CTA for an n-row system (0 if it does not fit 16 CTAs).
 int cluster_rows_for(int kind, int dtype, int64_t n, int requested);
 // Launches n_clusters clusters of csize CTAs that take systems from
-// d_queue (zero it first) until n_systems are done.
+// d_queue (zero it first) until n_systems are done.  slots > 0 (from
+// cluster_cg_slots): the slice-form CG kernel, with cluster_cg_workspace bytes
+// a CTA at `space`.
 int cluster_launch(const Handle &h, int kind, int dtype, bool jac, ClusterSystem *d_systems,
                    int n_systems, unsigned *d_queue, int rpc, int csize, int n_clusters,
-                   double budget_s, cudaStream_t stream, double delta = 0.0);
-int cluster_max_active(int kind, int dtype, bool jac, int rpc, int csize);
+                   double budget_s, cudaStream_t stream, double delta = 0.0, int slots = 0,
+                   void *space = nullptr);
+int cluster_max_active(int kind, int dtype, bool jac, int rpc, int csize, int slots = 0);
+// The slots a launch needs for systems whose longest row is longest_row, with
+// `rows` per CTA; 0 where the slice form does not apply (not CG, rows longer
+// than it takes, or no room for them).
+int cluster_cg_slots(int kind, int dtype, int rows, int longest_row);
+size_t cluster_cg_workspace(int dtype, int rows, int slots);
+int cluster_cg_launch(int dtype, bool jac, ClusterSystem *d_systems, int n_systems,
+                      unsigned *d_queue, int rpc, int csize, int n_clusters, double budget_s,
+                      cudaStream_t stream, int slots, void *space);
+int cluster_cg_max_active(int dtype, int rpc, int csize, int slots);
+// CG on all SMs in one cooperative launch: rows per CTA for an n-row system
+// (0 if it does not fit), its device workspace, and the launch.
+int grid_cg_rows(int dtype, int64_t n, int num_sms);
+size_t grid_cg_space(int dtype, int64_t n, int rows, int slots);
+int grid_cg_launch(const Handle &h, int dtype, bool jac, ClusterSystem *d_system, int64_t n,
+                   int rows, int slots, void *space, double budget_s, cudaStream_t stream);
 struct ServeRing;
 // The serving kernel (FP64, kServeRows rows per CTA) on n_clusters
 // clusters of csize CTAs, fed from `ring`.
 int cluster_serve_launch(const ServeRing &ring, int csize, int n_clusters, double budget_s,
                          cudaStream_t stream);
+
+// Whether a solve server exists in the process (mlsh_serve.cu): its persistent
+// kernels hold SMs for as long as requests keep coming, and a launch that
+// needs every SM at once would wait for them.
+bool server_running();
 
 // Mixed-precision data kept with an FP64 plan (mlsh_mixed.cu).
 void mixed_release(CsrPlan &p);

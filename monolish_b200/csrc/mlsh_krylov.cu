@@ -1236,19 +1236,35 @@ int ensure_ws(Handle &h, size_t bytes) {
 
 namespace {
 
-// One system on the cluster engine.  Returns MLSH_NOT_IMPL when the system
-// does not fit it (the caller then uses the kernel engine).
+// CG systems from this size on run on all SMs (one cooperative launch) rather
+// than on one cluster of at most 16: its barriers cost three times a
+// cluster's, but the rows are spread over up to nine times the SMs.  The line
+// lies where a cluster's CTAs pass 2,048 FP64 rows and their matrix no longer
+// fits shared memory: 32,761 rows 3.9 us per iteration on a cluster, 7.3 on all
+// SMs; 50,176 rows 7.6 and 7.3; 102,400 rows 16.0 and 8.1.
+constexpr int64_t kGridMinRows = 32769;
+
+// One system in one launch: on one cluster, or (grid) on all SMs.  Returns
+// MLSH_NOT_IMPL when the system does not fit (the caller then uses the
+// kernel engine).
 int cluster_solve_one(Kind kind, Handle &h, CsrPlan &p, const void *b, void *x,
-                      const mlsh_solver_opts *opts, mlsh_solver_result *res) {
+                      const mlsh_solver_opts *opts, mlsh_solver_result *res, bool grid) {
   const int64_t n = p.n_rows;
-  const int rpc = cluster_rows_for(kind == kCG ? 0 : 1, p.dtype, n, opts->cluster_rows);
+  const int rpc = grid ? grid_cg_rows(p.dtype, n, h.num_sms)
+                       : cluster_rows_for(kind == kCG ? 0 : 1, p.dtype, n, opts->cluster_rows);
   if (rpc == 0) return MLSH_NOT_IMPL;
+  const int slots = cluster_cg_slots(kind == kCG ? 0 : 1, p.dtype, rpc, p.longest_row);
+  if (grid && slots == 0) return MLSH_NOT_IMPL;
   const int csize = (int)((n + rpc - 1) / rpc);
   const bool jac = opts->precond == MLSH_PRECOND_JACOBI;
   const size_t esz = (size_t)dtype_size(p.dtype);
   const size_t vec = ((size_t)n * esz + 255) / 256 * 256;
-  // workspace: [system record][queue][inverse diagonal][r0]
-  int st = ensure_ws(h, 512 + 2 * vec);
+  // workspace: [system record][queue] and
+  //   cluster: [inverse diagonal][r0][matrix slices]
+  //   grid:    [sums and barriers][p][matrix slices]
+  int st = ensure_ws(h, 512 + (grid ? grid_cg_space(p.dtype, n, rpc, slots)
+                                    : 2 * vec + csize * cluster_cg_workspace(p.dtype, rpc,
+                                                                             slots)));
   if (st != MLSH_SUCCESS) return st;
   char *ws = static_cast<char *>(h.ws);
   ClusterSystem *d_sys = reinterpret_cast<ClusterSystem *>(ws);
@@ -1272,8 +1288,10 @@ int cluster_solve_one(Kind kind, Handle &h, CsrPlan &p, const void *b, void *x,
   hs->val = p.val;
   hs->b = b;
   hs->x = x;
-  hs->dinv = ws + 512;
-  hs->aux = ws + 512 + vec;
+  if (!grid) {
+    hs->dinv = ws + 512;
+    hs->aux = ws + 512 + vec;
+  }
   hs->n = (int)n;
   hs->tol = opts->tol;
   hs->maxiter = opts->maxiter;
@@ -1283,13 +1301,27 @@ int cluster_solve_one(Kind kind, Handle &h, CsrPlan &p, const void *b, void *x,
   hs->status = kRunning;
   MLSH_CUDA_TRY(cudaMemcpyAsync(d_sys, hs, sizeof(ClusterSystem), cudaMemcpyHostToDevice,
                                 h.stream));
-  MLSH_CUDA_TRY(cudaMemsetAsync(d_queue, 0, sizeof(unsigned), h.stream));
-  st = cluster_launch(h, kind == kCG ? 0 : 1, p.dtype, jac, d_sys, 1, d_queue, rpc, csize, 1,
-                      cluster_budget(opts), h.stream);
+  if (grid) {
+    MLSH_CUDA_TRY(cudaMemsetAsync(h.err_flag, 0, sizeof(int), h.stream));
+    st = grid_cg_launch(h, p.dtype, jac, d_sys, n, rpc, slots, ws + 512, cluster_budget(opts),
+                        h.stream);
+  } else {
+    MLSH_CUDA_TRY(cudaMemsetAsync(d_queue, 0, sizeof(unsigned), h.stream));
+    st = cluster_launch(h, kind == kCG ? 0 : 1, p.dtype, jac, d_sys, 1, d_queue, rpc, csize, 1,
+                        cluster_budget(opts), h.stream, 0.0, slots, ws + 512 + 2 * vec);
+  }
   if (st != MLSH_SUCCESS) return st;
   MLSH_CUDA_TRY(cudaMemcpyAsync(hs, d_sys, sizeof(ClusterSystem), cudaMemcpyDeviceToHost,
                                 h.stream));
+  if (grid)
+    MLSH_CUDA_TRY(cudaMemcpyAsync(&h.host_scalars[7], h.err_flag, sizeof(int),
+                                  cudaMemcpyDeviceToHost, h.stream));
   MLSH_CUDA_TRY(cudaStreamSynchronize(h.stream));
+  if (grid) {
+    int err = 0;
+    std::memcpy(&err, &h.host_scalars[7], sizeof(int));
+    if (err != 0) return err;
+  }
   res->status = hs->status;
   res->iters = hs->iters;
   res->final_resid = hs->resid;
@@ -1342,7 +1374,12 @@ int solve_common(Kind kind, mlsh_handle hs, mlsh_csr_plan ps, const void *b, voi
   }
   if (!pc && (opts->engine == MLSH_ENGINE_CLUSTER ||
               (opts->engine == MLSH_ENGINE_AUTO && opts->maxiter <= kClusterMaxIterAuto))) {
-    const int st = cluster_solve_one(kind, h, p, b, x, opts, res);
+    if (opts->engine == MLSH_ENGINE_AUTO && kind == kCG && n >= kGridMinRows &&
+        opts->cluster_rows <= 0 && !server_running()) {
+      const int gs = cluster_solve_one(kind, h, p, b, x, opts, res, true);
+      if (gs != MLSH_NOT_IMPL) return gs;
+    }
+    const int st = cluster_solve_one(kind, h, p, b, x, opts, res, false);
     if (st != MLSH_NOT_IMPL) return st;
     if (opts->engine == MLSH_ENGINE_CLUSTER) return MLSH_ERR_INVALID_ARG;
   }
