@@ -181,9 +181,11 @@ cudaError_t launch_spmv_t(const CsrPlan &p, const Handle &h, double alpha,
   a.err = h.err_flag;
   a.short_max = p.short_max;
   int v = p.variant;
-  // FP64 with two fused dots does not fit 4 CTAs per SM (56 registers: it
-  // spills); it runs the same pipeline depth at 3 CTAs per SM instead
-  if constexpr (sizeof(VT) == 8 && M0 != kDotNone && M1 != kDotNone) {
+  // FP64 with a weighted dot does not fit 4 CTAs per SM (56 registers: it
+  // spills 68-80 bytes a thread); it runs the same pipeline depth at 3 CTAs per
+  // SM instead.  With one weighted dot, us per iteration: CG on 101^3 rows 43.6
+  // at 4 CTAs, 38.3 at 3, on 128^3 79.5 and 70.6, BiCGSTAB on 160^3 298 and 292.
+  if constexpr (sizeof(VT) == 8 && M0 == kDotW) {
     static_assert(kSpmvVariants[2].min_blocks == 4 && kSpmvVariants[1].min_blocks == 3 &&
                       kSpmvVariants[1].stages == kSpmvVariants[2].stages,
                   "variant 1 is variant 2 at 3 CTAs per SM");
