@@ -553,7 +553,18 @@ int mlsh_csr_plan_create(mlsh_handle hs, int n_rows, int n_cols, int nnz,
     spmv_grids<double>(p.n_tiles, h.num_sms, p.spmv_grid);
   else
     spmv_grids<float>(p.n_tiles, h.num_sms, p.spmv_grid);
-  p.variant = kDefaultSpmvVariant;
+  // What the autotuner finds is the better start until it runs.  Rows of 9 to
+  // 16 entries go to one thread each as soon as there are any: a warp per such
+  // row spends most of its instructions on the tree.  FP64 rows far longer than
+  // the mean (columns scattered over x, the gathers' latency in front) gain
+  // from 3 CTAs per SM with three stages.  Zipf(2) rows, n = 4,194,304, FP64:
+  // 223 us at {2 stages, 4 CTAs} with limit 8, 219 with 16, 188 at {3, 3} with
+  // 16; the transpose of the one with 1,000,003 rows (rows of up to 22), FP32:
+  // 47 us with limit 8, 35 with 16, whatever the variant.
+  if (p.longest_row > kShortRow) p.short_max = 2 * kShortRow;
+  const bool uneven =
+      p.longest_row > kMaxShortRow && (int64_t)p.longest_row * n_rows > (int64_t)8 * nnz;
+  p.variant = dtype == MLSH_F64 && uneven ? 0 : kDefaultSpmvVariant;
   *out = ps;
   return MLSH_SUCCESS;
 }
