@@ -1359,13 +1359,22 @@ int build_dag(Handle &h, const int *rp, const int *ci, const int *lo, const int 
 // five or six CTAs of eight warps).
 constexpr int kSweepWarpsPerSm = 40;
 
-// Steps of a sweep: one per level, more where a level is wider than the
-// resident warps.
+// A block that the scan does not resolve runs a 32-step chain, and keeps its
+// sweep off the cluster: about three times a level of scans (24^3 rows in 41
+// such levels 283 us a sweep, in 70 levels of scans 112).
+constexpr double kChainSteps = 3.0;
+
+// Steps of a sweep: one per level of scan blocks, kChainSteps per level with
+// another block in it, more where a level is wider than the resident warps.
 double dag_steps(const BlockDag &d, int num_sms) {
   const double resident = (double)kSweepWarpsPerSm * num_sms;
+  std::vector<char> chain((size_t)d.levels, 0);
+  for (size_t b = 0; b < d.lvl.size(); ++b)
+    if (!d.scan[b]) chain[(size_t)d.lvl[b]] = 1;
   double steps = 0.0;
   for (int l = 0; l < d.levels; ++l)
-    steps += std::max(1.0, (d.level_off[(size_t)l + 1] - d.level_off[(size_t)l]) / resident);
+    steps += (chain[(size_t)l] ? kChainSteps : 1.0) *
+             std::max(1.0, (d.level_off[(size_t)l + 1] - d.level_off[(size_t)l]) / resident);
   return steps;
 }
 
@@ -1617,7 +1626,9 @@ __global__ void order_index_kernel(const SweepBlock *order, unsigned nb, int *or
 }
 
 // The cluster form of a sweep that would otherwise run over the whole GPU
-// through L2 flags: where a cluster (16 CTAs, else 8) can be resident with the
+// through L2 flags (49^3 rows: 2.3 us a level, on a cluster 1.6) or, levels too
+// wide for the ring, on one CTA with its rows loaded as it goes (24^3 rows: 6.8
+// us a level).  The ring (0.65 us a level, a few blocks wide) stays.  Where a cluster (16 CTAs, else 8) can be resident with the
 // solution in its shared memory, every block is resolved by the scan and no
 // row has more than four entries outside its block.
 template <typename T, int MODE>
@@ -1672,9 +1683,7 @@ int build_cluster_mode(Handle &h, const Precond &pc, const Sweep &sw, Schedule &
 
 template <typename T>
 int build_cluster_t(Handle &h, const Precond &pc, const Sweep &sw, Schedule &sc) {
-  if (sc.order == nullptr || pc.nb == 0 || sc.levels == 0 ||
-      cta_smem_bytes<T>(pc.n, pc.nb, sc.levels) <= kCtaSweepBytes)
-    return MLSH_SUCCESS;
+  if (sc.order == nullptr || pc.nb == 0 || sc.levels == 0 || sc.ring > 0) return MLSH_SUCCESS;
   switch (sw.mode) {
     case kSorFwd: return build_cluster_mode<T, kSorFwd>(h, pc, sw, sc);
     case kUnitFwd: return build_cluster_mode<T, kUnitFwd>(h, pc, sw, sc);
@@ -1784,6 +1793,7 @@ int mlsh_precond_sweep_form(mlsh_precond pc, int *lower, int *upper) {
   const Precond &p = pc->p;
   auto form = [&](const Schedule &sc) {
     if (sc.order == nullptr) return -1;
+    if (sc.ctas > 0) return MLSH_SWEEP_FLAGS;
     if (sc.ring > 0) return MLSH_SWEEP_RING;
     const size_t bytes = p.dtype == MLSH_F64 ? cta_smem_bytes<double>(p.n, p.nb, sc.levels)
                                              : cta_smem_bytes<float>(p.n, p.nb, sc.levels);
