@@ -286,7 +286,8 @@ int mlsh_fill(mlsh_handle handle, int dtype, int64_t n, double value,
  *            wall-clock budget of 60 s per solve ends a solve that does not
  *            terminate with MLSH_ERR_TIMEOUT.
  *   AUTO     CLUSTER when the system fits and maxiter <= 2,000,000, else
- *            KERNELS.  CG of 32,769 rows and more, up to 4,096 FP64 or
+ *            KERNELS.  CG of 32,769 rows and more (65,537
+ *            when no row has more than 5 entries), up to 4,096 FP64 or
  *            8,192 FP32 rows an SM (606,208 / 1,212,416 on 148 SMs; rows of
  *            up to 16 entries): the same single launch over
  *            the whole GPU (a cooperative launch with the CLUSTER budget),

@@ -1073,10 +1073,15 @@ void destroy_entry(GraphEntry &e) {
 // Iterations in the while node's body: each pass of the node costs about two
 // launches (kernels of the iterations after the last one return at once,
 // st->done).  us per iteration with one and with eight: CG on 64^3 rows 24.4 and
-// 22.2, on 101^3 38.3 and 36.2, on 128^3 70.6 and 67.2.  BiCGSTAB keeps one: on
-// 160^3 292 with one, 314 with eight.
-constexpr int kBodyItersCg = 8;
-int body_iters(Kind kind) { return kind == kCG ? kBodyItersCg : 1; }
+// 22.2, on 101^3 38.3 and 36.2, on 128^3 70.6 and 67.2; BiCGSTAB on 48^3 37.2
+// and 34.5, on 101^3 84.3 and 83.3, but on 160^3 292 and 314: large BiCGSTAB
+// systems keep one.
+constexpr int kBodyIters = 8;
+constexpr int64_t kBodyItersMaxBicgstab = 2000000;
+int body_iters(Kind kind, int64_t n) {
+  if (kind == kCG || (kind == kBiCGSTAB && n <= kBodyItersMaxBicgstab)) return kBodyIters;
+  return 1;
+}
 
 // Builds  [init kernels] -> WHILE(cond) { body_iters iterations }  as one graph.
 int build_graph(const SolveCtx &c, Handle &h, GraphEntry &out) {
@@ -1168,7 +1173,7 @@ int build_graph(const SolveCtx &c, Handle &h, GraphEntry &out) {
       if (e == cudaSuccess) e = capture(ip.conditional.phGraph_out[0], mixbi_update, c2);
     }
   } else {
-    e = capture(body, iter, c, body_iters(c.kind));
+    e = capture(body, iter, c, body_iters(c.kind, c.n));
   }
   if (e != cudaSuccess) {
     cudaGraphDestroy(g);
@@ -1252,11 +1257,11 @@ namespace {
 
 // CG systems from this size on run on all SMs (one cooperative launch) rather
 // than on one cluster of at most 16: its barriers cost three times a
-// cluster's, but the rows are spread over up to nine times the SMs.  The line
-// lies where a cluster's CTAs pass 2,048 FP64 rows and their matrix no longer
-// fits shared memory: 32,761 rows 3.9 us per iteration on a cluster, 7.3 on all
-// SMs; 50,176 rows 7.6 and 7.3; 102,400 rows 16.0 and 8.1.
-constexpr int64_t kGridMinRows = 32769;
+// cluster's, but the rows are spread over up to nine times the SMs.  us per
+// iteration on a cluster / on all SMs, rows of 5 entries: 32,761 rows 3.8 / 7.3,
+// 65,536 rows 6.7 / 7.5, 68,644 rows (8,192 a CTA) 14.4 / 7.5; of 7 entries:
+// 32,768 rows 4.8 / 9.2, 46,656 rows 8.2 / 7.8, 68,921 rows 16.7 / 7.9.
+int64_t grid_min_rows(int longest_row) { return longest_row <= 5 ? 65537 : 32769; }
 
 // One system in one launch: on one cluster, or (grid) on all SMs.  Returns
 // MLSH_NOT_IMPL when the system does not fit (the caller then uses the
@@ -1388,7 +1393,7 @@ int solve_common(Kind kind, mlsh_handle hs, mlsh_csr_plan ps, const void *b, voi
   }
   if (!pc && (opts->engine == MLSH_ENGINE_CLUSTER ||
               (opts->engine == MLSH_ENGINE_AUTO && opts->maxiter <= kClusterMaxIterAuto))) {
-    if (opts->engine == MLSH_ENGINE_AUTO && kind == kCG && n >= kGridMinRows &&
+    if (opts->engine == MLSH_ENGINE_AUTO && kind == kCG && n >= grid_min_rows(p.longest_row) &&
         opts->cluster_rows <= 0 && !server_running()) {
       const int gs = cluster_solve_one(kind, h, p, b, x, opts, res, true);
       if (gs != MLSH_NOT_IMPL) return gs;

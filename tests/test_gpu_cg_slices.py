@@ -77,7 +77,7 @@ def check(handle, restatement, mat, dtype=np.float64, precond=_abi.PRECOND_JACOB
 
 # rows: one CTA and its edges, cluster slices of 1,024 / 2,048 rows with a last
 # CTA of one row and of all, the last size on a cluster, the first on the GPU
-@pytest.mark.parametrize("n", [1, 31, 33, 1023, 1025, 16384, 16385, 32768, 32769, 40001])
+@pytest.mark.parametrize("n", [1, 31, 33, 1023, 1025, 16384, 16385, 32768, 32769, 65536, 65537])
 def test_sizes(handle, restatement, n):
     nx = max(1, int(np.sqrt(n)))
     while n % nx:
@@ -101,14 +101,14 @@ def test_whole_gpu_3d(handle, restatement, m, dtype):
     check(handle, restatement, shifted(*W.vardiff3d(m, m, m, 3, 0)[1:], 0.7), dtype)
 
 
-@pytest.mark.parametrize("n", [2500, 50000])
+@pytest.mark.parametrize("n", [2500, 70000])
 @pytest.mark.parametrize("width", [1, 4, 7, 8])
 def test_row_lengths(handle, restatement, n, width):
     """Rows of up to 3, 9, 15 and 17 entries (the last in the row-loop form)."""
     check(handle, restatement, banded(n, width, width))
 
 
-@pytest.mark.parametrize("n", [900, 48400])
+@pytest.mark.parametrize("n", [900, 72900])
 def test_no_preconditioner_and_initial_guess(handle, restatement, n):
     m = int(np.sqrt(n))
     check(handle, restatement, shifted(*W.poisson2d(m, m)[1:], 0.5),
@@ -120,7 +120,7 @@ def test_whole_gpu_stops(handle):
     a repeat gives the same bits; beside a server the kernel engine solves."""
     import torch
     from monolish_b200 import device as D
-    n, rp, ci, v = W.poisson2d(210, 200)
+    n, rp, ci, v = W.poisson2d(310, 300)
     A = D.Crs(handle, n, n, rp, ci, v)
     b = torch.ones(n, dtype=torch.float64, device="cuda")
     x = torch.zeros_like(b)
