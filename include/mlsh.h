@@ -204,7 +204,10 @@ int mlsh_spmv_transpose(mlsh_handle handle, mlsh_csr_plan plan, double alpha,
  * count left.  Replaces COO::sort(merge)
  * (src/utils/at_insert_sort/at_insert_sort_coo.cpp:119-145), whose
  * quicksort leaves the order of duplicates unspecified.  Indices outside
- * [0,n_rows) x [0,n_cols) give MLSH_ERR_INVALID_ARG. */
+ * [0,n_rows) x [0,n_cols) give MLSH_ERR_INVALID_ARG.  Scratch of up to 1 GiB
+ * (about 16 bytes per entry and 8 per row, 36 per entry from 4 million entries
+ * on) stays with the handle, as the solvers' work vectors do; more is released
+ * before the call returns.  mlsh_csr_transpose likewise. */
 int mlsh_coo_sort(mlsh_handle handle, int n_rows, int n_cols, int64_t nnz, int *d_row,
                   int *d_col, void *d_val, int dtype, int merge, int64_t *new_nnz);
 

@@ -44,7 +44,7 @@ struct SortFlags {
   int bad;              // an index was out of range
   unsigned longest;     // entries of the largest group
   unsigned n_long;      // groups over kSegCap
-  unsigned kept;        // entries left after merging
+  unsigned far;         // sampled warps whose entries' rows lie far apart
 };
 
 // Where the ordered entries go (null: not wanted).

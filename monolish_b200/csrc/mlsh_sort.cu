@@ -239,6 +239,8 @@ __global__ void lower_bounds(const unsigned *keys, long long n, int n_out, int *
 constexpr int kGroupItems = 4;
 
 // Entries per key (and the range check of both indices; `other` may be null).
+// One warp in four also says whether its 32 entries are spread over more than
+// 1/64 of the keys.
 __global__ void __launch_bounds__(256) count_keys(const int *key, const int *other, long long n,
                                                   int n_keys, int n_other, unsigned *cnt,
                                                   SortFlags *flags) {
@@ -250,6 +252,12 @@ __global__ void __launch_bounds__(256) count_keys(const int *key, const int *oth
     k[u] = i < n ? key[i] : 0;
     o[u] = i < n && other ? other[i] : 0;
   }
+  const unsigned active = __ballot_sync(0xffffffffu, base < n);
+  const int span = active == 0xffffffffu ? __reduce_max_sync(0xffffffffu, k[0]) -
+                                               __reduce_min_sync(0xffffffffu, k[0])
+                                         : 0;
+  const int far = __syncthreads_count((threadIdx.x & 31) == 0 && span > n_keys / 64);
+  if (threadIdx.x == 0 && far > 0) atomicAdd(&flags->far, (unsigned)far);
 #pragma unroll
   for (int u = 0; u < kGroupItems; ++u) {
     if (base + u * 256 >= n) break;
@@ -287,6 +295,81 @@ __global__ void __launch_bounds__(256) scatter_coo(const int *row, const int *co
       x[u] = SortRec<T>{col[i], (unsigned)i, val[i]};
     }
   }
+#pragma unroll
+  for (int u = 0; u < kGroupItems; ++u)
+    if (base + u * 256 < n) rec[atomicAdd(cursor + r[u], 1u)] = x[u];
+}
+
+// ---- entries in no order, more of them than L2 holds: two scatters
+// Every 16-byte store of scatter_coo then opens a line of its own in HBM.  The
+// entries go first to 256 ranges of rows, whose records fill the same place
+// there as they will in the end (about 1/256 of the array: the second scatter's
+// stores meet in L2).  16.1 M shuffled triplets, sorted and converted: 1.52 ms
+// with one scatter (672 us of it), 1.31 with two.  A CTA collects its entries by range in shared memory and
+// writes each range's run contiguously.
+constexpr int kRangeItems = 8;
+constexpr int kRangeTile = 256 * kRangeItems;
+
+// Where each range starts: the first row's start (starts is the scanned count).
+__global__ void __launch_bounds__(256) range_starts(const unsigned *starts, int n_keys, int shift,
+                                                    unsigned n, unsigned *cursor) {
+  const long long row = (long long)threadIdx.x << shift;
+  cursor[threadIdx.x] = row < n_keys ? starts[row] : n;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) ranges_coo(const int *row, const int *col, const T *val,
+                                                  long long n, int shift, unsigned *cursor,
+                                                  SortRec<T> *rec, int *rec_row) {
+  __shared__ SortRec<T> s_rec[kRangeTile];
+  __shared__ int s_row[kRangeTile];
+  __shared__ unsigned s_cnt[256], s_local[256], s_to[256], s_warp[kSortWarps];
+  const int t = threadIdx.x;
+  const long long base = (long long)blockIdx.x * kRangeTile + t;
+  s_cnt[t] = 0;
+  __syncthreads();
+  int r[kRangeItems];
+  unsigned rank[kRangeItems];
+#pragma unroll
+  for (int u = 0; u < kRangeItems; ++u) r[u] = base + u * 256 < n ? row[base + u * 256] : -1;
+#pragma unroll
+  for (int u = 0; u < kRangeItems; ++u)
+    if (r[u] >= 0) rank[u] = atomicAdd(&s_cnt[r[u] >> shift], 1u);
+  __syncthreads();
+  unsigned total;
+  s_local[t] = block_exclusive_scan(s_cnt[t], s_warp, &total);
+  s_to[t] = s_cnt[t] > 0 ? atomicAdd(cursor + t, s_cnt[t]) : 0u;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kRangeItems; ++u)
+    if (r[u] >= 0) {
+      const long long i = base + u * 256;
+      const unsigned at = s_local[r[u] >> shift] + rank[u];
+      s_rec[at] = SortRec<T>{col[i], (unsigned)i, val[i]};
+      s_row[at] = r[u];
+    }
+  __syncthreads();
+  for (unsigned k = t; k < total; k += 256) {
+    const int b = s_row[k] >> shift;
+    const unsigned to = s_to[b] + (k - s_local[b]);
+    rec[to] = s_rec[k];
+    rec_row[to] = s_row[k];
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) scatter_ranges(const SortRec<T> *in, const int *in_row,
+                                                      long long n, unsigned *cursor,
+                                                      SortRec<T> *rec) {
+  const long long base = (long long)blockIdx.x * (256 * kGroupItems) + threadIdx.x;
+  int r[kGroupItems];
+  SortRec<T> x[kGroupItems];
+#pragma unroll
+  for (int u = 0; u < kGroupItems; ++u)
+    if (base + u * 256 < n) {
+      r[u] = in_row[base + u * 256];
+      x[u] = in[base + u * 256];
+    }
 #pragma unroll
   for (int u = 0; u < kGroupItems; ++u)
     if (base + u * 256 < n) rec[atomicAdd(cursor + r[u], 1u)] = x[u];
@@ -506,16 +589,21 @@ struct GroupScratch {
   unsigned *sums = nullptr;
   unsigned *long_ids = nullptr;
   void *rec = nullptr;
+  void *rec2 = nullptr;        // ranges: the entries by range of rows, their rows,
+  int *row2 = nullptr;
+  unsigned *ranges = nullptr;  // and the ranges' cursors
   void *own = nullptr;
   cudaStream_t s = nullptr;
 
-  int alloc(Handle &h, long long n, long long n_keys) {
+  int alloc(Handle &h, long long n, long long n_keys, bool two_scatters) {
     s = h.stream;
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t keys_b = up(sizeof(unsigned) * (size_t)n_keys);
     const size_t sums_b = up(sizeof(unsigned) * (size_t)(sort_tiles(n_keys) + 1));
     const size_t long_b = up(sizeof(unsigned) * (size_t)(n / kSegCap + 1));
-    const size_t total = 256 + 2 * keys_b + sums_b + long_b + 16 * (size_t)n;
+    const size_t rec_b = up(16 * (size_t)n);
+    const size_t one = 256 + 2 * keys_b + sums_b + long_b + rec_b;
+    const size_t total = one + (two_scatters ? rec_b + up(4 * (size_t)n) + 1024 : 0);
     char *p = nullptr;
     if (total <= kKeepScratch) {
       const int st = ensure_ws(h, total);
@@ -535,6 +623,11 @@ struct GroupScratch {
     sums = reinterpret_cast<unsigned *>(p + 256 + 2 * keys_b);
     long_ids = reinterpret_cast<unsigned *>(p + 256 + 2 * keys_b + sums_b);
     rec = p + 256 + 2 * keys_b + sums_b + long_b;
+    if (two_scatters) {
+      rec2 = p + one;
+      row2 = reinterpret_cast<int *>(p + one + rec_b);
+      ranges = reinterpret_cast<unsigned *>(p + one + rec_b + up(4 * (size_t)n));
+    }
     return MLSH_SUCCESS;
   }
   ~GroupScratch() {
@@ -544,6 +637,10 @@ struct GroupScratch {
     }
   }
 };
+
+// Records of more than this take two scatters when their rows are in no order:
+// below it the destinations stay in L2 anyway.
+constexpr long long kTwoScatterBytes = 64ll << 20;
 
 // Keys far more numerous than entries: counting and scanning them would cost
 // more than sorting the entries.
@@ -630,7 +727,8 @@ int coo_group_sort(Handle &h, int n_rows, int n_cols, long long n, int *row, int
                    bool merge, long long *total, bool *done) {
   *done = false;
   GroupScratch w;
-  int st = w.alloc(h, n, n_rows);
+  const bool large = 16 * n >= kTwoScatterBytes;
+  int st = w.alloc(h, n, n_rows, large);
   if (st != MLSH_SUCCESS) return st;
   SortFlags f;
   st = count_groups(w, h, row, col, n, n_rows, n_cols, &f);
@@ -639,8 +737,18 @@ int coo_group_sort(Handle &h, int n_rows, int n_cols, long long n, int *row, int
   if (f.longest > (unsigned)kLongCap) return MLSH_SUCCESS;
   *done = true;
   scan_exclusive(w.ends, w.ends, n_rows, w.sums, w.s);
-  scatter_coo<T><<<group_blocks(n), 256, 0, w.s>>>(row, col, val, n, w.ends,
-                                                   static_cast<SortRec<T> *>(w.rec));
+  auto *rec = static_cast<SortRec<T> *>(w.rec);
+  if (large && (long long)f.far * 64 > n / kGroupItems) {  // more than half the sampled warps
+    int shift = 0;
+    while ((n_rows - 1) >> shift > 255) ++shift;
+    auto *rec2 = static_cast<SortRec<T> *>(w.rec2);
+    range_starts<<<1, 256, 0, w.s>>>(w.ends, n_rows, shift, (unsigned)n, w.ranges);
+    ranges_coo<T><<<(unsigned)((n + kRangeTile - 1) / kRangeTile), 256, 0, w.s>>>(
+        row, col, val, n, shift, w.ranges, rec2, w.row2);
+    scatter_ranges<T><<<group_blocks(n), 256, 0, w.s>>>(rec2, w.row2, n, w.ends, rec);
+  } else {
+    scatter_coo<T><<<group_blocks(n), 256, 0, w.s>>>(row, col, val, n, w.ends, rec);
+  }
   return order_all<T>(w, h, n, n_rows, f.longest, merge, SortOut<T>{row, col, val, nullptr},
                       total);
 }
@@ -652,7 +760,7 @@ int transpose_group(Handle &h, int n_rows, int n_cols, long long nnz, const int 
                     unsigned *perm_out, bool *done) {
   *done = false;
   GroupScratch w;
-  int st = w.alloc(h, nnz, n_cols);
+  int st = w.alloc(h, nnz, n_cols, false);
   if (st != MLSH_SUCCESS) return st;
   SortFlags f;
   st = count_groups(w, h, ci, nullptr, nnz, n_cols, 0, &f);
@@ -872,7 +980,7 @@ int mlsh_coo_sort(mlsh_handle hs, int n_rows, int n_cols, int64_t nnz, int *d_ro
   // By counting where no row is longer than the ordering kernels take and the
   // rows are not far more than the entries; the radix sort otherwise.  Sort,
   // merge and row pointers of 16.1 M shuffled triplets of the 128^3 7-point
-  // matrix (FP64): 1.52 ms, by the radix sort 13.1 ms; the transpose of the
+  // matrix (FP64): 1.31 ms, by the radix sort 13.1 ms; the transpose of the
   // 1,000,003-row Zipf(2) matrix with its first product 7.4 against 14.6 ms.
   int st = MLSH_SUCCESS;
   if (groups_worth(n, n_rows)) {

@@ -95,3 +95,29 @@ def test_sort_between_solves(handle):
     D.coo_sort(handle, 20000, 5000, _dev(row), _dev(col), _dev(val))
     assert torch.equal(x1, solve())
     A.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n_rows", [300, 65537, 4000000])
+@pytest.mark.parametrize("k,order", [((1 << 22) - 1, "shuffled"), ((1 << 22) + 777, "shuffled"),
+                                     ((1 << 22) + 777, "rows")])
+def test_two_scatters(handle, n_rows, k, order, dtype):
+    """Entries in no order, just below and above the size from which they go to
+    ranges of rows first, and in row order (one scatter); against numpy."""
+    from monolish_b200 import device as D
+    rng = np.random.default_rng(k + n_rows)
+    row = rng.integers(0, n_rows, k, dtype=np.int32)
+    if order == "rows":
+        row.sort()
+    # few columns in long rows, so that entries repeat
+    col = rng.integers(0, 3 if n_rows > 1000 else 20000, k, dtype=np.int32)
+    val = rng.uniform(-1, 1, k).astype(dtype)
+    o = np.lexsort((np.arange(k), col, row))
+    last = np.ones(k, bool)
+    last[:-1] = (row[o][1:] != row[o][:-1]) | (col[o][1:] != col[o][:-1])
+    dr, dc, dv = _dev(row), _dev(col), _dev(val)
+    cnt = D.coo_sort(handle, n_rows, 20000, dr, dc, dv, merge=True)
+    assert cnt == int(last.sum())
+    assert np.array_equal(dr.cpu().numpy()[:cnt], row[o][last])
+    assert np.array_equal(dc.cpu().numpy()[:cnt], col[o][last])
+    assert np.array_equal(dv.cpu().numpy()[:cnt], val[o][last])
