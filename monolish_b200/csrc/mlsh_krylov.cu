@@ -1074,10 +1074,11 @@ void destroy_entry(GraphEntry &e) {
 // launches (kernels of the iterations after the last one return at once,
 // st->done).  us per iteration with one and with eight: CG on 64^3 rows 24.4 and
 // 22.2, on 101^3 38.3 and 36.2, on 128^3 70.6 and 67.2; BiCGSTAB on 48^3 37.2
-// and 34.5, on 101^3 84.3 and 83.3, but on 160^3 292 and 314: large BiCGSTAB
-// systems keep one.
+// and 34.5, on 101^3 84.3 and 83.3, but on 160^3 292 and 314.  A BiCGSTAB solve
+// with one and with eight: 105^3 17.9 and 18.2 ms, 112^3 22.1 and 22.9, 124^3 30.9
+// and 33.2: systems of more than 1.1 M rows keep one.
 constexpr int kBodyIters = 8;
-constexpr int64_t kBodyItersMaxBicgstab = 2000000;
+constexpr int64_t kBodyItersMaxBicgstab = 1100000;
 int body_iters(Kind kind, int64_t n) {
   if (kind == kCG || (kind == kBiCGSTAB && n <= kBodyItersMaxBicgstab)) return kBodyIters;
   return 1;
