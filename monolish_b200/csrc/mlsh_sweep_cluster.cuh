@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kClSweepThreads, 1)
   namespace cgs = cooperative_groups;
   cgs::cluster_group cl = cgs::this_cluster();
   extern __shared__ __align__(16) unsigned char sweep_cluster_smem[];
-  __shared__ uint64_t level_bar;
+  __shared__ uint64_t level_bar[2];  // levels take them in turn (see below)
   __shared__ int s_late;
   if (a.done != nullptr && *(volatile const int *)a.done != 0) return;  // all CTAs alike
   const int ctas = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -185,9 +185,10 @@ __global__ void __launch_bounds__(kClSweepThreads, 1)
   T *xs = reinterpret_cast<T *>(sweep_cluster_smem);
   int *s_loff = reinterpret_cast<int *>(sweep_cluster_smem + (size_t)most * 32 * sizeof(T));
   for (int i = threadIdx.x; i <= a.levels; i += kClSweepThreads) s_loff[i] = a.level_off[i];
-  const uint32_t bar = smem_addr(&level_bar);
+  const uint32_t bar0 = smem_addr(level_bar);
   if (threadIdx.x == 0) {
-    mbar_init(bar, (uint32_t)ctas);
+    mbar_init(bar0, (uint32_t)ctas);
+    mbar_init(bar0 + 8, (uint32_t)ctas);
     s_late = 0;
     fence_mbar_init();
   }
@@ -217,7 +218,14 @@ __global__ void __launch_bounds__(kClSweepThreads, 1)
       }
     }
     if (lv + 1 == a.levels) break;
-    // this CTA's part of the level is written: tell every CTA, wait for all
+    // This CTA's part of the level is written: tell every CTA, wait for all.
+    // Arrivals carry no sender and remote ones reach different CTAs in any
+    // order, so with one barrier a CTA that has left level lv could fill, with
+    // its arrival for lv + 1, the place of one still under way for lv.  With
+    // two, the next arrival on this barrier is for lv + 2: its sender has seen
+    // everybody arrive for lv + 1, which a CTA does once it has left lv.
+    const uint32_t bar = bar0 + 8u * ((uint32_t)lv & 1u);
+    const uint32_t phase = ((uint32_t)lv >> 1) & 1u;
     __syncthreads();
     if ((int)threadIdx.x < ctas) {
       uint32_t to;
@@ -228,7 +236,7 @@ __global__ void __launch_bounds__(kClSweepThreads, 1)
     bool ok = true;
     if (warp == 0) {  // one warp asks, the others wait behind it
       ok = false;
-      for (unsigned p = 0; p < a.polls && !ok; ++p) ok = mbar_test_cluster(bar, (uint32_t)lv & 1u);
+      for (unsigned p = 0; p < a.polls && !ok; ++p) ok = mbar_test_cluster(bar, phase);
       if (!ok) s_late = 1;
     }
     if (__syncthreads_or(ok ? 0 : 1)) break;
