@@ -339,7 +339,9 @@ int batch_run(Handle &h, Batch &B, int kind, const void *d_b, void *d_x, const d
   int first_bad = MLSH_SUCCESS;
   for (int i = 0; i < B.n_systems; ++i) {
     const int k = order[i];
-    const ClusterSystem &S = B.h_sys[i];
+    ClusterSystem &S = B.h_sys[i];
+    // left in the queue by clusters that gave up on a wait
+    if (S.status == kRunning) S.status = MLSH_ERR_TIMEOUT;
     if (host_status) host_status[k] = S.status;
     if (host_iters) host_iters[k] = S.iters;
     if (host_resid) host_resid[k] = S.resid;

@@ -163,7 +163,7 @@ int grid_cg_launch(const Handle &h, int dtype, bool jac, ClusterSystem *d_system
   c.space = p;
   c.space_bytes = cluster_cg_workspace(dtype, rows, slots);
   c.err = h.err_flag;
-  MLSH_CUDA_TRY(cudaMemsetAsync(space, 0, sizeof(unsigned), stream));
+  MLSH_CUDA_TRY(cudaMemsetAsync(space, 0, 2 * sizeof(unsigned), stream));  // count, late
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;

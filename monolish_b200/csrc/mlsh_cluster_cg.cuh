@@ -106,7 +106,8 @@ inline size_t cg_space_bytes(int esz, int rows, int slots) {
 // What the CTAs of a whole-GPU launch exchange.
 struct GridSpace {
   unsigned count;  // arrivals, zero before the launch
-  unsigned pad[31];
+  unsigned late;   // set once a CTA's wait gave up, zero before the launch
+  unsigned pad[30];
   double part[2][2][kMaxGridCtas];
   double flag[2];
 };
@@ -190,9 +191,15 @@ __device__ __forceinline__ void cta_sum2(CgShared &sh, double &a, double &b) {
   b = __shfl_sync(0xffffffffu, v, 16);
 }
 
+// What a CTA whose wait gave up sends for its partials: a NaN that no sum
+// comes out as.  Whoever reads it among the partials knows that this sum, and
+// everything since that wait, holds nothing.
+constexpr unsigned long long kLatePartial = 0x7ff81a7e1a7e1a7eull;
+
 // The CTAs of one cluster as the solve sees them.  A wait that gives up sets
-// sh.late; the CTA then leaves the solve and meets the others at the
-// hardware barrier that ends it (nobody leaves while messages may arrive).
+// sh.late, which stays set: the CTA sends kLatePartial from then on, so every
+// CTA leaves the solve at its next sum, and they meet at the hardware barrier
+// that ends it (nobody leaves while messages may arrive).
 struct ClusterTeam {
   static constexpr bool kGrid = false;
   cooperative_groups::cluster_group &cl;
@@ -201,6 +208,17 @@ struct ClusterTeam {
   unsigned n_sums, n_bars;  // so far: which barrier and phase comes next
   __device__ void start() { cl.sync(); }
   __device__ void finish() { cl.sync(); }
+  // Between two solves: whether a wait gave up in any CTA (the same answer in
+  // all of them).  The barriers' phases hold nothing then.
+  __device__ bool any_late() {
+    int l = 0;
+    if (threadIdx.x < size)
+      asm volatile("ld.shared::cluster.s32 %0, [%1];"
+                   : "=r"(l)
+                   : "r"(map_cluster(smem_addr(&sh.late), threadIdx.x))
+                   : "memory");
+    return __syncthreads_or(l) != 0;
+  }
   // Every thread's p is written and everyone may read it.
   __device__ void barrier() {
     __syncthreads();
@@ -210,8 +228,8 @@ struct ClusterTeam {
     if (!wait_for([&] { return mbar_try_wait_cluster(bar, ph); })) sh.late = 1;
   }
   // Sums of a and b over the team and thread 0 of CTA 0's `flag` (2 after a
-  // wait gave up), in warp 0.  The partials are added in a fixed tree, so all
-  // CTAs hold identical values.
+  // wait gave up in any CTA), in warp 0.  The partials are added in a fixed
+  // tree, so all CTAs hold identical values.
   __device__ void sums(double &a, double &b, double &flag) {
     const int lane = threadIdx.x & 31;
     const unsigned par = n_sums & 1u, ph = (n_sums >> 1) & 1u;
@@ -221,6 +239,7 @@ struct ClusterTeam {
     const uint32_t bar = smem_addr(&sh.sum_bar[par]);
     const double f = __shfl_sync(0xffffffffu, flag, 0);
     if (lane == 0) mbar_arrive_expect_tx(bar, size * 16u + 8u);
+    if (sh.late != 0) a = b = __longlong_as_double((long long)kLatePartial);
     if ((unsigned)lane < size) {
       const uint32_t to = map_cluster(bar, lane);
       st_async(map_cluster(smem_addr(&sh.part[par][2 * rank]), lane), a, b, to);
@@ -228,7 +247,10 @@ struct ClusterTeam {
     }
     const bool ok = wait_for([&] { return mbar_try_wait_cluster(bar, ph); });
     double v = (unsigned)(lane & 15) < size ? sh.part[par][2 * (lane & 15) + (lane >> 4)] : 0.0;
-    flag = ok && sh.late == 0 ? sh.flag[par] : 2.0;
+    const bool lost = !ok || (unsigned long long)__double_as_longlong(v) == kLatePartial;
+    if (lost) sh.late = 1;
+    __syncwarp();
+    flag = sh.late == 0 ? sh.flag[par] : 2.0;
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     a = __shfl_sync(0xffffffffu, v, 0);
@@ -254,7 +276,8 @@ struct ClusterTeam {
 // All CTAs of a cooperative launch.  p is also kept in global memory, where
 // other CTAs read it through L2; sums and barriers go through an arrival
 // counter there, which one thread per CTA polls (all threads polling words of
-// their own made a sum three times slower).  Waits are bounded as above.
+// their own made a sum three times slower).  Waits are bounded as above; a CTA
+// whose wait gave up sets space->late before it arrives again.
 struct GridTeam {
   static constexpr bool kGrid = true;
   CgShared &sh;
@@ -267,6 +290,7 @@ struct GridTeam {
   // One thread: release this CTA's writes (ordered before it by the CTA
   // barrier or the warp), arrive, wait for the others' arrivals.
   __device__ bool meet() {
+    if (sh.late != 0) atomicExch(&space->late, 1u);
     __threadfence();
     atomicAdd(&space->count, 1u);
     const unsigned want = n_bars * size;
@@ -284,15 +308,14 @@ struct GridTeam {
     ++n_bars;
     cta_sum2(sh, a, b);
     if (threadIdx.x >= 32) return;
-    int ok = 1;
     if (lane == 0) {
       space->part[par][0][rank] = a;
       space->part[par][1][rank] = b;
       if (rank == 0) space->flag[par] = flag;
-      ok = meet() ? 1 : 0;
-      if (!ok) sh.late = 1;
+      if (!meet()) sh.late = 1;
     }
-    ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();  // the other lanes' reads come after lane 0's meeting
+    const bool lost = sh.late != 0 || __ldcg(&space->late) != 0;
     // CTA c in lane c % 32, then a tree
     double va = 0.0, vb = 0.0;
     for (unsigned c = lane; c < size; c += 32) {
@@ -303,7 +326,7 @@ struct GridTeam {
     const double v = warp_sum2(va, vb, lane);
     a = __shfl_sync(0xffffffffu, v, 0);
     b = __shfl_sync(0xffffffffu, v, 16);
-    flag = ok && sh.late == 0 ? f : 2.0;
+    flag = lost ? 2.0 : f;
   }
   template <typename T>
   __device__ void publish(int row, T v) {
@@ -688,6 +711,10 @@ __global__ void __launch_bounds__(kCgThreads, 1) cluster_cg_kernel(const CgArgs 
     const unsigned long long idx = sh.sys_idx;
     if (idx >= (unsigned long long)a.n_systems) break;
     cg_solve_slices<T, RT>(team, a, a.systems[idx], cg_smem, ring_at);
+    if (team.any_late()) {  // the other clusters take what is left in the queue
+      cl.sync();
+      break;
+    }
   }
 }
 
