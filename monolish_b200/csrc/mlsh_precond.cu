@@ -70,8 +70,9 @@ __global__ void split_rows_kernel(const int *rp, const int *ci, int n, int *lo_e
                                   int *up_beg, int *bad, unsigned long long *missing,
                                   unsigned *links) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int b = rp[i], e = rp[i + 1];
+  // threads past the end keep an empty row: the ballots below take whole warps
+  const bool in = i < n;
+  const int b = in ? rp[i] : 0, e = in ? rp[i + 1] : 0;
   int lo = e, up = e, prev = -1;
   for (int j = b; j < e; ++j) {
     const int c = ci[j];
@@ -80,16 +81,18 @@ __global__ void split_rows_kernel(const int *rp, const int *ci, int n, int *lo_e
     if (lo == e && c >= i) lo = j;
     if (up == e && c > i) up = j;
   }
-  lo_end[i] = lo;
-  up_beg[i] = up;
-  if (up == lo) atomicMin(missing, (unsigned long long)i);
+  if (in) {
+    lo_end[i] = lo;
+    up_beg[i] = up;
+    if (up == lo) atomicMin(missing, (unsigned long long)i);
+  }
   if (links != nullptr) {
     // lanes hold consecutive rows: one OR per warp and word (the upper link
     // of row i is row i + 1's bit)
-    const unsigned act = __activemask();
     const bool lower = lo > b && ci[lo - 1] == i - 1;
     const bool upper = up < e && ci[up] == i + 1;
-    const unsigned m = __ballot_sync(act, lower) | (__ballot_sync(act, upper) << 1);
+    const unsigned m =
+        __ballot_sync(0xffffffffu, lower) | (__ballot_sync(0xffffffffu, upper) << 1);
     if ((i & 31) == 0 && m != 0) atomicOr(links + (i >> 5), m);
     if ((i & 31) == 31 && upper) atomicOr(links + (i >> 5) + 1, 1u);
   }

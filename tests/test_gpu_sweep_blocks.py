@@ -96,3 +96,41 @@ def test_odd_lines(handle, restatement, name, dtype):
         assert err < (1e-12 if dtype == np.float64 else 1e-5), (kind, err)
         pc.close()
     A.close()
+
+
+def host_blocks(rp, ci):
+    """Blocks cut at 32 rows and where a row and the one before it do not
+    depend on each other."""
+    n = len(rp) - 1
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    linked = np.zeros(n + 1, bool)
+    linked[rows[ci == rows - 1]] = True
+    linked[rows[ci == rows + 1] + 1] = True
+    blocks, rows_in = 0, 32
+    for i in range(n):
+        if rows_in == 32 or not linked[i]:
+            blocks, rows_in = blocks + 1, 0
+        rows_in += 1
+    return blocks
+
+
+@pytest.mark.parametrize("line,lines", [(33, 61), (40, 50), (63, 9)])
+def test_blocks_of_uneven_rows(handle, line, lines):
+    """Links between rows are found whatever the rows' lengths are: every
+    seventh row also has entries in the first line's columns, and the last
+    warp has rows past the end."""
+    from monolish_b200 import device as D
+    _, rp, ci, v = W.poisson2d(line, lines)
+    n = len(rp) - 1
+    rng = np.random.default_rng(2)
+    cols = [ci[rp[i]:rp[i + 1]] for i in range(n)]
+    for i in range(2 * line, n, 7):
+        cols[i] = np.union1d(cols[i], rng.choice(line, int(rng.integers(1, line)), replace=False))
+    rp = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.int32)
+    ci = np.concatenate(cols).astype(np.int32)
+    A = D.Crs(handle, n, n, rp, ci, np.where(np.repeat(np.arange(n), np.diff(rp)) == ci, 99.0, -1))
+    for _ in range(3):
+        pc = D.Precond(A, SOR, omega=1.0)
+        assert pc.info()[2] == host_blocks(rp, ci)
+        pc.close()
+    A.close()
