@@ -21,7 +21,7 @@
 
 namespace mlsh {
 
-constexpr int kMaxBatchGroups = 128;
+constexpr int kMaxBatchGroups = 256;  // 16 cluster sizes, 5 slice widths, 2 kernels
 constexpr int kMaxRowsPerCta = 16384;  // the widest slice the engine takes
 constexpr int kMinRowsPerCta = 1024;
 
@@ -56,8 +56,9 @@ struct Batch {
   ClusterSystem *h_sys = nullptr;     // pinned mirror
   unsigned *d_queue = nullptr;        // one counter per group
   void *ws = nullptr;                 // inverse diagonal + BiCGSTAB r0
-  int *d_longest = nullptr;           // longest row of each system
-  std::vector<int> longest;
+  int64_t *d_row_off = nullptr;       // row_off on the device
+  int *d_longest = nullptr;           // CG: longest row of each system, as the
+  std::vector<int> longest;           // last solve found it (empty before one)
   void *space = nullptr;              // CG: the groups' matrix slices
   size_t space_bytes = 0;
   cudaEvent_t done_event = nullptr;
@@ -68,13 +69,16 @@ namespace {
 // Groups for one kind: systems by needed cluster size (largest first).
 // Each system takes the widest slice (rows per CTA, a power of two up to
 // B.rpc_cap[kind]) that fits the engine; when none under the cap fits, the
-// narrowest that does.
+// narrowest that does.  CG systems whose own longest row is past the slice
+// form go to groups of their own: which kernel solves a system depends on that
+// system alone.
 int build_groups(Batch &B, int kind, std::vector<BatchGroup> &groups,
                  std::vector<int> &order) {
   const int cap = B.rpc_cap[kind];
   const int n = B.n_systems;
   const int dt = kind == 2 ? MLSH_F32 : B.dtype;  // mixed CG iterates in FP32
   std::vector<int> rpc(n), cs(n);
+  std::vector<char> loops(n, 0);  // CG: solved by the row-loop kernel
   for (int k = 0; k < n; ++k) {
     const int64_t nk = B.row_off[k + 1] - B.row_off[k];
     // one CTA while the system fits one; otherwise the widest slices
@@ -95,12 +99,15 @@ int build_groups(Batch &B, int kind, std::vector<BatchGroup> &groups,
     rpc[k] = r;
     cs[k] = (int)((nk + r - 1) / r);
     if (cs[k] < 1) cs[k] = 1;
+    if (kind == 0 && !B.longest.empty())
+      loops[k] = cluster_cg_slots(kind, dt, r, B.longest[(size_t)k]) == 0 ? 1 : 0;
   }
   order.resize(n);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     if (cs[a] != cs[b]) return cs[a] > cs[b];
     if (rpc[a] != rpc[b]) return rpc[a] > rpc[b];
+    if (loops[a] != loops[b]) return loops[a] < loops[b];
     const int64_t na = B.row_off[a + 1] - B.row_off[a];
     const int64_t nb = B.row_off[b + 1] - B.row_off[b];
     return na > nb;
@@ -108,7 +115,8 @@ int build_groups(Batch &B, int kind, std::vector<BatchGroup> &groups,
   groups.clear();
   for (int i = 0; i < n; ++i) {
     const int k = order[i];
-    if (groups.empty() || groups.back().csize != cs[k] || groups.back().rpc != rpc[k]) {
+    if (groups.empty() || groups.back().csize != cs[k] || groups.back().rpc != rpc[k] ||
+        loops[order[i - 1]] != loops[k]) {
       if ((int)groups.size() == kMaxBatchGroups) return MLSH_ERR_INVALID_ARG;
       BatchGroup g;
       g.csize = cs[k];
@@ -141,16 +149,18 @@ void free_batch(Batch &B) {
   cudaFree(B.d_queue);
   cudaFree(B.ws);
   cudaFree(B.val32);
+  cudaFree(B.d_row_off);
   cudaFree(B.d_longest);
   cudaFree(B.space);
   if (B.done_event) cudaEventDestroy(B.done_event);
 }
 
-// Longest row of system blockIdx.x; row_off[k] is where system k's rows start.
-__global__ void __launch_bounds__(256) longest_rows(const ClusterSystem *sys, int *out) {
-  const int *rp = sys[blockIdx.x].rp;
+// Longest row of system blockIdx.x, whose rows are row_off[k] .. row_off[k + 1].
+__global__ void __launch_bounds__(256)
+    longest_rows(const int *rp, const int64_t *row_off, int *out) {
   int m = 0;
-  for (int i = threadIdx.x; i < sys[blockIdx.x].n; i += 256) m = max(m, rp[i + 1] - rp[i]);
+  for (int64_t i = row_off[blockIdx.x] + threadIdx.x; i < row_off[blockIdx.x + 1]; i += 256)
+    m = max(m, rp[i + 1] - rp[i]);
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0) atomicMax(out + blockIdx.x, m);
 }
@@ -208,6 +218,10 @@ int mlsh_batch_create(mlsh_handle hs, int n_systems, const int64_t *row_off,
             cudaMallocHost(&B.h_sys, sizeof(ClusterSystem) * n_rec) == cudaSuccess &&
             cudaMalloc(&B.d_queue, sizeof(unsigned) * kMaxBatchGroups) == cudaSuccess &&
             cudaMalloc(&B.d_longest, sizeof(int) * n_rec) == cudaSuccess &&
+            cudaMalloc(&B.d_row_off, sizeof(int64_t) * (n_rec + 1)) == cudaSuccess &&
+            (n_systems == 0 ||
+             cudaMemcpy(B.d_row_off, row_off, sizeof(int64_t) * ((size_t)n_systems + 1),
+                        cudaMemcpyHostToDevice) == cudaSuccess) &&
             cudaMalloc(&B.ws, 2 * esz * (size_t)std::max<int64_t>(B.total_rows, 1) + 256) ==
                 cudaSuccess &&
             cudaEventCreateWithFlags(&B.done_event, cudaEventDisableTiming) == cudaSuccess;
@@ -234,6 +248,23 @@ int mlsh_batch_destroy(mlsh_batch bs) {
 namespace mlsh {
 namespace {
 
+// The longest row of each system (read anew for every solve: the caller owns
+// the row pointers); CG systems are grouped by it.
+int read_longest(Handle &h, Batch &B) {
+  MLSH_CUDA_TRY(cudaMemsetAsync(B.d_longest, 0, sizeof(int) * B.n_systems, h.stream));
+  longest_rows<<<(unsigned)B.n_systems, 256, 0, h.stream>>>(B.row_ptr, B.d_row_off, B.d_longest);
+  MLSH_CUDA_TRY(cudaGetLastError());
+  std::vector<int> now((size_t)B.n_systems);
+  MLSH_CUDA_TRY(cudaMemcpyAsync(now.data(), B.d_longest, sizeof(int) * B.n_systems,
+                                cudaMemcpyDeviceToHost, h.stream));
+  MLSH_CUDA_TRY(cudaStreamSynchronize(h.stream));
+  if (now != B.longest) {
+    B.longest.swap(now);
+    drop_groups(B, 0);
+  }
+  return MLSH_SUCCESS;
+}
+
 // One batched solve of `kind` (0 CG, 1 BiCGSTAB, 2 mixed CG with refresh
 // factor `delta`).
 int batch_run(Handle &h, Batch &B, int kind, const void *d_b, void *d_x, const double *host_tol,
@@ -243,6 +274,10 @@ int batch_run(Handle &h, Batch &B, int kind, const void *d_b, void *d_x, const d
   if (!d_b || !d_x) return MLSH_ERR_INVALID_ARG;
   std::vector<BatchGroup> &groups = B.groups[kind];
   std::vector<int> &order = B.order[kind];
+  if (kind == 0) {
+    const int st = read_longest(h, B);
+    if (st != MLSH_SUCCESS) return st;
+  }
   if (groups.empty()) {
     const int st = build_groups(B, kind, groups, order);
     if (st != MLSH_SUCCESS) return st;
@@ -280,23 +315,15 @@ int batch_run(Handle &h, Batch &B, int kind, const void *d_b, void *d_x, const d
                                 cudaMemcpyHostToDevice, h.stream));
   MLSH_CUDA_TRY(cudaMemsetAsync(B.d_queue, 0, sizeof(unsigned) * kMaxBatchGroups, h.stream));
   const int n_groups = (int)groups.size();
-  // CG: the longest row of each group decides its kernel and its workspace
-  // (read anew each time: the caller owns the row pointers)
-  if (kind == 0) {
-    MLSH_CUDA_TRY(cudaMemsetAsync(B.d_longest, 0, sizeof(int) * B.n_systems, h.stream));
-    longest_rows<<<(unsigned)B.n_systems, 256, 0, h.stream>>>(B.d_sys, B.d_longest);
-    MLSH_CUDA_TRY(cudaGetLastError());
-    B.longest.resize((size_t)B.n_systems);
-    MLSH_CUDA_TRY(cudaMemcpyAsync(B.longest.data(), B.d_longest, sizeof(int) * B.n_systems,
-                                  cudaMemcpyDeviceToHost, h.stream));
-    MLSH_CUDA_TRY(cudaStreamSynchronize(h.stream));
-  }
+  // CG: a group's slices are as wide as its longest row; the groups of longer
+  // rows, whose systems do not fit the form, get 0 slots
   size_t space = 0;
   for (BatchGroup &g : groups) {
     g.slots = 0;
     if (kind == 0) {
       int m = 0;
-      for (int i = g.first; i < g.first + g.count; ++i) m = std::max(m, B.longest[(size_t)i]);
+      for (int i = g.first; i < g.first + g.count; ++i)
+        m = std::max(m, B.longest[(size_t)order[(size_t)i]]);
       g.slots = cluster_cg_slots(kind, dt, g.rpc, m);
     }
     g.n_clusters = cluster_max_active(kind, dt, jac, g.rpc, g.csize, g.slots);

@@ -219,3 +219,34 @@ def test_batch_repeats_bitwise(handle, restatement):
             assert np.array_equal(got[1], first[1]) and np.array_equal(got[2], first[2])
             assert np.array_equal(got[0], first[0])
     B.close()
+
+
+def test_long_row_beside(handle, restatement):
+    """Which kernel solves a system is its own affair: beside one with a row of
+    17 entries (past the slice form) and the same rows per CTA and cluster size,
+    a system gives the bits that it gives alone, and so does the other."""
+    rng = np.random.default_rng(3)
+    rp, ci, v = make_systems([3000], seed=29)[0]
+    long_rp, long_ci, long_v = make_systems([2900], seed=31)[0]
+    n = len(long_rp) - 1
+    row = n // 2  # symmetric: the extra columns' rows get one entry each
+    rows = [dict(zip(long_ci[long_rp[i]:long_rp[i + 1]], long_v[long_rp[i]:long_rp[i + 1]]))
+            for i in range(n)]
+    for j in rng.choice(np.setdiff1d(np.arange(n), list(rows[row])), 17 - len(rows[row]),
+                        replace=False):
+        w = -0.01 * rng.random()
+        for a, b in ((row, int(j)), (int(j), row)):
+            rows[a][b] = w
+            rows[a][a] += abs(w)
+    assert max(len(r) for r in rows) == 17
+    long_system = (np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32),
+                   np.concatenate([sorted(r) for r in rows]).astype(np.int32),
+                   np.concatenate([[r[c] for c in sorted(r)] for r in rows]))
+    systems = [(rp, ci, v), long_system]
+    status, iters, _, xs, _, _ = run_batch(handle, systems, "cg", 1e-8, 5000, restatement)
+    assert (status == 0).all()
+    for k in range(2):
+        s1, i1, _, x1, _, _ = run_batch(handle, [systems[k]], "cg", 1e-8, 5000, restatement,
+                                        x_seed=5 + k)
+        assert (s1[0], i1[0]) == (0, iters[k])
+        assert np.array_equal(x1[0], xs[k])
