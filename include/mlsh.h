@@ -288,16 +288,22 @@ int mlsh_fill(mlsh_handle handle, int dtype, int64_t n, double value,
  *            (CG, FP64) / 65,536 (BiCGSTAB, FP64), twice that in FP32.  A
  *            wall-clock budget of 60 s per solve ends a solve that does not
  *            terminate with MLSH_ERR_TIMEOUT.
+ *   GRID     CG only: the whole solve in one cooperative launch over all
+ *            SMs, with the CLUSTER budget.  For a caller that has the GPU to
+ *            itself: the launch waits until every SM is free, so it follows
+ *            whatever else runs (a batch, another thread's solve) and can
+ *            starve beside a busy solve server.  Up to 4,096 FP64 or 8,192
+ *            FP32 rows an SM (606,208 / 1,212,416 on 148 SMs) with rows of up
+ *            to 12 (FP32: 16) entries, 16 in FP64 too up to 1,024 rows an SM;
+ *            anything else runs as KERNELS.
+ *            Faster than CLUSTER from about 65,537 rows (5 entries a row) or
+ *            32,769 rows (7) on.
  *   AUTO     CLUSTER when the system fits and maxiter <= 2,000,000, else
- *            KERNELS.  CG of 32,769 rows and more (65,537
- *            when no row has more than 5 entries), up to 4,096 FP64 or
- *            8,192 FP32 rows an SM (606,208 / 1,212,416 on 148 SMs; rows of
- *            up to 16 entries): the same single launch over
- *            the whole GPU (a cooperative launch with the CLUSTER budget),
- *            unless a solve server runs in the process. */
+ *            KERNELS. */
 #define MLSH_ENGINE_AUTO 0
 #define MLSH_ENGINE_KERNELS 1
 #define MLSH_ENGINE_CLUSTER 2
+#define MLSH_ENGINE_GRID 3
 
 typedef struct {
   double tol;       /* absolute threshold on ||r||_2, like solver::set_tol

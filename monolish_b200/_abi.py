@@ -50,6 +50,7 @@ class SolverOpts(C.Structure):
 ENGINE_AUTO = 0
 ENGINE_KERNELS = 1
 ENGINE_CLUSTER = 2
+ENGINE_GRID = 3
 
 
 class SolverResult(C.Structure):

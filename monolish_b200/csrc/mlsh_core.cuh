@@ -72,11 +72,6 @@ struct ServeRing;
 int cluster_serve_launch(const ServeRing &ring, int csize, int n_clusters, double budget_s,
                          cudaStream_t stream);
 
-// Whether a solve server exists in the process (mlsh_serve.cu): its persistent
-// kernels hold SMs for as long as requests keep coming, and a launch that
-// needs every SM at once would wait for them.
-bool server_running();
-
 // Mixed-precision data kept with an FP64 plan (mlsh_mixed.cu).
 void mixed_release(CsrPlan &p);
 void mixed_invalidate(CsrPlan &p);

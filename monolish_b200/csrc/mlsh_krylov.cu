@@ -1256,14 +1256,6 @@ int ensure_ws(Handle &h, size_t bytes) {
 
 namespace {
 
-// CG systems from this size on run on all SMs (one cooperative launch) rather
-// than on one cluster of at most 16: its barriers cost three times a
-// cluster's, but the rows are spread over up to nine times the SMs.  us per
-// iteration on a cluster / on all SMs, rows of 5 entries: 32,761 rows 3.8 / 7.3,
-// 65,536 rows 6.7 / 7.5, 68,644 rows (8,192 a CTA) 14.4 / 7.5; of 7 entries:
-// 32,768 rows 4.8 / 9.2, 46,656 rows 8.2 / 7.8, 68,921 rows 16.7 / 7.9.
-int64_t grid_min_rows(int longest_row) { return longest_row <= 5 ? 65537 : 32769; }
-
 // One system in one launch: on one cluster, or (grid) on all SMs.  Returns
 // MLSH_NOT_IMPL when the system does not fit (the caller then uses the
 // kernel engine).
@@ -1392,13 +1384,20 @@ int solve_common(Kind kind, mlsh_handle hs, mlsh_csr_plan ps, const void *b, voi
     }
     return res->status;
   }
+  // All SMs (one cooperative launch) only when the caller asks for it: the
+  // launch takes every SM, so solves of several threads that would run side by
+  // side on clusters of 16 follow one another, and beside a busy server it may
+  // wait without end.  Its barriers cost three times a cluster's, but the rows
+  // are spread over up to nine times the SMs.  us per iteration on a cluster /
+  // on all SMs, rows of 5 entries: 32,761 rows 3.8 / 7.3, 65,536 rows 6.7 / 7.5,
+  // 68,644 rows (8,192 a CTA) 14.4 / 7.5; of 7 entries: 32,768 rows 4.8 / 9.2,
+  // 46,656 rows 8.2 / 7.8, 68,921 rows 16.7 / 7.9.
+  if (!pc && kind == kCG && opts->engine == MLSH_ENGINE_GRID) {
+    const int gs = cluster_solve_one(kind, h, p, b, x, opts, res, true);
+    if (gs != MLSH_NOT_IMPL) return gs;
+  }
   if (!pc && (opts->engine == MLSH_ENGINE_CLUSTER ||
               (opts->engine == MLSH_ENGINE_AUTO && opts->maxiter <= kClusterMaxIterAuto))) {
-    if (opts->engine == MLSH_ENGINE_AUTO && kind == kCG && n >= grid_min_rows(p.longest_row) &&
-        opts->cluster_rows <= 0 && !server_running()) {
-      const int gs = cluster_solve_one(kind, h, p, b, x, opts, res, true);
-      if (gs != MLSH_NOT_IMPL) return gs;
-    }
     const int st = cluster_solve_one(kind, h, p, b, x, opts, res, false);
     if (st != MLSH_NOT_IMPL) return st;
     if (opts->engine == MLSH_ENGINE_CLUSTER) return MLSH_ERR_INVALID_ARG;

@@ -38,12 +38,6 @@
 namespace mlsh {
 
 namespace {
-std::atomic<int> g_servers{0};
-}
-
-bool server_running() { return g_servers.load(std::memory_order_relaxed) > 0; }
-
-namespace {
 
 constexpr unsigned kRingCapacity = 1024;
 constexpr int kRingClasses = 2;                       // 1-CTA and 16-CTA clusters
@@ -495,7 +489,6 @@ int mlsh_server_create(size_t budget, int n_lanes, mlsh_server *out) {
     delete ss;
     return st;
   }
-  g_servers.fetch_add(1, std::memory_order_relaxed);
   S.sched = std::thread(scheduler, &S);
   for (int i = 0; i < n_lanes; ++i) S.lanes.emplace_back(lane_worker, &S);
   *out = ss;
@@ -596,7 +589,6 @@ int mlsh_server_destroy(mlsh_server ss) {
   if (S.down) cudaStreamDestroy(S.down);
   for (auto &kv : S.all) delete kv.second;
   delete ss;
-  g_servers.fetch_sub(1, std::memory_order_relaxed);
   return MLSH_SUCCESS;
 }
 
