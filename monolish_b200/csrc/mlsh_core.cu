@@ -60,11 +60,12 @@ void build_tiles(const int *rp, int n_rows, std::vector<Tile> &tiles,
   }
 }
 
-// Every (type, dot modes, variant) instantiation of the SpMV kernel.
-template <typename VT, int M0, int M1, int V, bool C16 = false>
+// Every (type, dot modes, variant) instantiation of the SpMV kernel; the
+// kernels with TREE sum rows of 9 .. 16 entries in one thread.
+template <typename VT, int M0, int M1, int V, bool C16 = false, bool TREE = false>
 static constexpr auto spmv_kernel_ptr() {
   return spmv_tiles_kernel<VT, VT, M0, M1, kSpmvVariants[V].stages, kSpmvVariants[V].min_blocks,
-                           C16>;
+                           C16, TREE>;
 }
 
 template <typename VT, int V, bool C16 = false>
@@ -72,31 +73,27 @@ static constexpr int spmv_smem_bytes() {
   return SpmvSmem<VT, kSpmvVariants[V].stages, C16 ? 2 : 4>::kBytes;
 }
 
-template <typename VT, int M0, int M1, int V, bool C16 = false>
-static int set_spmv_smem_one() {
-  const cudaError_t e = cudaFuncSetAttribute(spmv_kernel_ptr<VT, M0, M1, V, C16>(),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             spmv_smem_bytes<VT, V, C16>());
-  if (e != cudaSuccess) {
-    set_last_error("cudaFuncSetAttribute(spmv)", e);
-    return MLSH_ERR_CUDA;
-  }
+template <typename VT, int M0, int M1, bool C16, bool TREE, int... V>
+static int set_spmv_smem_all(std::integer_sequence<int, V...>) {
+  for (const cudaError_t e :
+       {cudaFuncSetAttribute(spmv_kernel_ptr<VT, M0, M1, V, C16, TREE>(),
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             spmv_smem_bytes<VT, V, C16>())...})
+    if (e != cudaSuccess) {
+      set_last_error("cudaFuncSetAttribute(spmv)", e);
+      return MLSH_ERR_CUDA;
+    }
   return MLSH_SUCCESS;
 }
 
 template <typename VT, int M0, int M1>
 static int set_spmv_smem() {
-  int s = set_spmv_smem_one<VT, M0, M1, 0>();
-  if (s == MLSH_SUCCESS) s = set_spmv_smem_one<VT, M0, M1, 1>();
-  if (s == MLSH_SUCCESS) s = set_spmv_smem_one<VT, M0, M1, 2>();
-  if (s == MLSH_SUCCESS) s = set_spmv_smem_one<VT, M0, M1, 3>();
-  if (s == MLSH_SUCCESS) s = set_spmv_smem_one<VT, M0, M1, 4>();
+  constexpr auto all = std::make_integer_sequence<int, kNumSpmvVariants>{};
+  int s = set_spmv_smem_all<VT, M0, M1, false, false>(all);
+  if (s == MLSH_SUCCESS) s = set_spmv_smem_all<VT, M0, M1, false, true>(all);
   if constexpr (sizeof(VT) == 4) {
-    if (s == MLSH_SUCCESS) s = set_spmv_smem_one<VT, M0, M1, 0, true>();
-    if (s == MLSH_SUCCESS) s = set_spmv_smem_one<VT, M0, M1, 1, true>();
-    if (s == MLSH_SUCCESS) s = set_spmv_smem_one<VT, M0, M1, 2, true>();
-    if (s == MLSH_SUCCESS) s = set_spmv_smem_one<VT, M0, M1, 3, true>();
-    if (s == MLSH_SUCCESS) s = set_spmv_smem_one<VT, M0, M1, 4, true>();
+    if (s == MLSH_SUCCESS) s = set_spmv_smem_all<VT, M0, M1, true, false>(all);
+    if (s == MLSH_SUCCESS) s = set_spmv_smem_all<VT, M0, M1, true, true>(all);
   }
   return s;
 }
@@ -149,6 +146,28 @@ static void spmv_grids(int n_tiles, int num_sms, int *grid) {
 }
 
 // ------------------------------------------------------- SpMV launcher --
+template <typename VT, int M0, int M1, bool C16, bool TREE>
+static cudaError_t launch_spmv_variant(int v, int grid, cudaStream_t stream,
+                                       const SpmvArgs<VT, VT> &a) {
+  switch (v) {
+    case 1:
+      return launch_dependent(spmv_kernel_ptr<VT, M0, M1, 1, C16, TREE>(), grid, kSpmvThreads,
+                              spmv_smem_bytes<VT, 1, C16>(), stream, a);
+    case 2:
+      return launch_dependent(spmv_kernel_ptr<VT, M0, M1, 2, C16, TREE>(), grid, kSpmvThreads,
+                              spmv_smem_bytes<VT, 2, C16>(), stream, a);
+    case 3:
+      return launch_dependent(spmv_kernel_ptr<VT, M0, M1, 3, C16, TREE>(), grid, kSpmvThreads,
+                              spmv_smem_bytes<VT, 3, C16>(), stream, a);
+    case 4:
+      return launch_dependent(spmv_kernel_ptr<VT, M0, M1, 4, C16, TREE>(), grid, kSpmvThreads,
+                              spmv_smem_bytes<VT, 4, C16>(), stream, a);
+    default:
+      return launch_dependent(spmv_kernel_ptr<VT, M0, M1, 0, C16, TREE>(), grid, kSpmvThreads,
+                              spmv_smem_bytes<VT, 0, C16>(), stream, a);
+  }
+}
+
 template <typename VT, int M0, int M1>
 cudaError_t launch_spmv_t(const CsrPlan &p, const Handle &h, double alpha,
                           const VT *x, double beta, const VT *y_in, VT *y_out,
@@ -196,60 +215,19 @@ cudaError_t launch_spmv_t(const CsrPlan &p, const Handle &h, double alpha,
     if (v == 4) v = 0;
   }
   const int g = p.spmv_grid[v];
-  cudaError_t e = cudaSuccess;
+  // rows of 9 .. 16 entries as the warp adds them, unless the limit has them in
+  // row order anyway
+  const bool tree = p.short_max == kShortRow && p.longest_row > kShortRow;
   if constexpr (sizeof(VT) == 4) {
     if (p.slots != nullptr)
       return launch_spmv_slots<M0, M1>(p, h, alpha, x, beta, y_in, y_out, w0, w1, dot_out,
                                        done, stream);
-    if (p.col16 != nullptr) {
-      switch (v) {
-        case 1:
-          e = launch_dependent(spmv_kernel_ptr<VT, M0, M1, 1, true>(), g, kSpmvThreads,
-                               spmv_smem_bytes<VT, 1, true>(), stream, a);
-          break;
-        case 2:
-          e = launch_dependent(spmv_kernel_ptr<VT, M0, M1, 2, true>(), g, kSpmvThreads,
-                               spmv_smem_bytes<VT, 2, true>(), stream, a);
-          break;
-        case 3:
-          e = launch_dependent(spmv_kernel_ptr<VT, M0, M1, 3, true>(), g, kSpmvThreads,
-                               spmv_smem_bytes<VT, 3, true>(), stream, a);
-          break;
-        case 4:
-          e = launch_dependent(spmv_kernel_ptr<VT, M0, M1, 4, true>(), g, kSpmvThreads,
-                               spmv_smem_bytes<VT, 4, true>(), stream, a);
-          break;
-        default:
-          e = launch_dependent(spmv_kernel_ptr<VT, M0, M1, 0, true>(), g, kSpmvThreads,
-                               spmv_smem_bytes<VT, 0, true>(), stream, a);
-          break;
-      }
-      return e;
-    }
+    if (p.col16 != nullptr)
+      return tree ? launch_spmv_variant<VT, M0, M1, true, true>(v, g, stream, a)
+                  : launch_spmv_variant<VT, M0, M1, true, false>(v, g, stream, a);
   }
-  switch (v) {
-    case 1:
-      e = launch_dependent(spmv_kernel_ptr<VT, M0, M1, 1>(), g, kSpmvThreads,
-                           spmv_smem_bytes<VT, 1>(), stream, a);
-      break;
-    case 2:
-      e = launch_dependent(spmv_kernel_ptr<VT, M0, M1, 2>(), g, kSpmvThreads,
-                           spmv_smem_bytes<VT, 2>(), stream, a);
-      break;
-    case 3:
-      e = launch_dependent(spmv_kernel_ptr<VT, M0, M1, 3>(), g, kSpmvThreads,
-                           spmv_smem_bytes<VT, 3>(), stream, a);
-      break;
-    case 4:
-      e = launch_dependent(spmv_kernel_ptr<VT, M0, M1, 4>(), g, kSpmvThreads,
-                           spmv_smem_bytes<VT, 4>(), stream, a);
-      break;
-    default:
-      e = launch_dependent(spmv_kernel_ptr<VT, M0, M1, 0>(), g, kSpmvThreads,
-                           spmv_smem_bytes<VT, 0>(), stream, a);
-      break;
-  }
-  return e;
+  return tree ? launch_spmv_variant<VT, M0, M1, false, true>(v, g, stream, a)
+              : launch_spmv_variant<VT, M0, M1, false, false>(v, g, stream, a);
 }
 
 #define MLSH_INST_SPMV(VT, A, B)                                                 \
@@ -553,15 +531,10 @@ int mlsh_csr_plan_create(mlsh_handle hs, int n_rows, int n_cols, int nnz,
     spmv_grids<double>(p.n_tiles, h.num_sms, p.spmv_grid);
   else
     spmv_grids<float>(p.n_tiles, h.num_sms, p.spmv_grid);
-  // What the autotuner finds is the better start until it runs.  Rows of 9 to
-  // 16 entries go to one thread each as soon as there are any: a warp per such
-  // row spends most of its instructions on the tree.  FP64 rows far longer than
-  // the mean (columns scattered over x, the gathers' latency in front) gain
-  // from 3 CTAs per SM with three stages.  Zipf(2) rows, n = 4,194,304, FP64:
-  // 223 us at {2 stages, 4 CTAs} with limit 8, 219 with 16, 188 at {3, 3} with
-  // 16; the transpose of the one with 1,000,003 rows (rows of up to 22), FP32:
-  // 47 us with limit 8, 35 with 16, whatever the variant.
-  if (p.longest_row > kShortRow) p.short_max = 2 * kShortRow;
+  // What the autotuner finds is the better start until it runs.  FP64 rows far
+  // longer than the mean (columns scattered over x, the gathers' latency in
+  // front) gain from 3 CTAs per SM with three stages: Zipf(2) rows, n =
+  // 4,194,304, FP64, 219 us at {2 stages, 4 CTAs}, 188 at {3, 3}.
   const bool uneven =
       p.longest_row > kMaxShortRow && (int64_t)p.longest_row * n_rows > (int64_t)8 * nnz;
   p.variant = dtype == MLSH_F64 && uneven ? 0 : kDefaultSpmvVariant;

@@ -28,6 +28,11 @@
 //              bit-identical to it);
 //      longer rows: the whole warp, one such row after another (lane-
 //              strided partial sums, then an xor tree) -- deterministic;
+//              with the limit at 8, rows of 9 to 16 entries take the same
+//              tree in one thread, with the same bits (TREE): Zipf(2) rows, n
+//              = 4,194,304, FP64, variant {2, 4}: 165 us, by warps 206, in row
+//              order (limit 16) 200; the transpose of 1,000,003 such rows,
+//              FP32: 28.4 us, in row order 27.2, by warps 41
 //      then y is written coalesced and the fused dots accumulate in a
 //      fixed per-thread order.  Each thread's row bounds, dot weight and
 //      the tile's column base for the next tile are fetched one tile ahead.
@@ -101,6 +106,12 @@ constexpr int kFlagConsAbort = 1;
 constexpr int kFlagLast = 3;
 constexpr int kFlagWarpDone = 4;  // 8 slots: tiles each consumer warp has consumed
 
+constexpr int kTreeRow = 16;
+// The tree's order of eight even entries (see the kernel).
+__device__ __forceinline__ constexpr int tree_entry(int u) {
+  return (int)((0xe6a2c480u >> (4 * u)) & 15u);
+}
+
 template <typename T>
 __device__ __forceinline__ T spmv_mul_rn(T a, T b) {
   if constexpr (sizeof(T) == 8) return __dmul_rn(a, b);
@@ -137,7 +148,10 @@ __device__ __forceinline__ uint32_t rounded_range(const E *arr, int nb, int ne, 
 // C16: columns stored as 16-bit offsets from a per-tile base (2 bytes per
 // nonzero instead of 4) -- the plan picks it when every tile's columns span
 // fewer than 65,536 values.
-template <typename VT, typename XT, int M0, int M1, int STAGES, int MINB, bool C16 = false>
+// TREE: rows of up to kTreeRow entries by one thread (for plans with rows of 9
+// entries and more and a short-row limit of 8).
+template <typename VT, typename XT, int M0, int M1, int STAGES, int MINB, bool C16 = false,
+          bool TREE = false>
 __global__ void __launch_bounds__(kSpmvThreads, MINB)
     spmv_tiles_kernel(const SpmvArgs<VT, XT> a) {
   constexpr int NR = (M0 != kDotNone ? 1 : 0) + (M1 != kDotNone ? 1 : 0);
@@ -363,11 +377,50 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
       //    separately rounded products -- the reference's loop, so these
       //    rows are bit-identical to it;
       //  * longer rows: the whole warp, one row after another (lane-strided
-      //    partial sums, then an xor tree), the owning thread keeps the sum.
+      //    partial sums, then an xor tree), the owning thread keeps the sum;
+      //  * TREE: rows of 9 .. 16 entries by one thread in the order of that
+      //    tree, a few operations instead of a warp's shuffles per row.  Row
+      //    order would do as few, but its rounding errors add up to 1.17x (9
+      //    entries) to 1.35x (16) the tree's.
       VT sum = VT(0);
       const int s0 = g0 - nb, len = g1 - g0;
-      const int smax = a.short_max;
-      if (ct < nrows && len <= smax) {
+      const int smax = TREE ? kTreeRow : a.short_max;
+      if constexpr (TREE) {
+        if (ct < nrows && len <= kTreeRow) {
+          // Entries in two rounds of eight gathers; rows of up to 8 need one
+          // and are added in row order.  Lane l of the xor tree adds entries l
+          // and l + 8, then l + 4's sum, l + 2's, l + 1's: round 0 takes the
+          // even entries (lane 0's sum) as 0, 8, 4, 12, 2, 10, 6, 14, round 1
+          // the odd ones (lane 1's).  Absent entries are zeros, as there.
+          const bool tree = len > kShortRow;
+          for (int r = 0; r < (tree ? 2 : 1); ++r) {
+            XT xx[kShortRow];
+#pragma unroll
+            for (int u = 0; u < kShortRow; ++u) {
+              const int k = tree ? r + tree_entry(u) : u;
+              xx[u] = k < len ? __ldg(a.x + col_at(s0 + k)) : XT(0);
+            }
+            if (tree) {
+              VT half[2];
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                VT q[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  const int k = r + tree_entry(4 * h + u);
+                  q[u] = k < len ? spmv_mul_rn(v[s0 + k], (VT)xx[4 * h + u]) : VT(0);
+                }
+                half[h] = spmv_add_rn(spmv_add_rn(q[0], q[1]), spmv_add_rn(q[2], q[3]));
+              }
+              sum = spmv_add_rn(sum, spmv_add_rn(half[0], half[1]));
+            } else {
+#pragma unroll
+              for (int u = 0; u < kShortRow; ++u)
+                if (u < len) sum = spmv_add_rn(sum, spmv_mul_rn(v[s0 + u], (VT)xx[u]));
+            }
+          }
+        }
+      } else if (ct < nrows && len <= smax) {
         // kShortRow gathers in flight at a time; the sum stays in row order
         for (int u0 = 0; u0 < len; u0 += kShortRow) {
           XT xx[kShortRow];

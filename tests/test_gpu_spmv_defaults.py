@@ -1,6 +1,7 @@
 """The SpMV variant and short-row limit a plan starts with: rows up to the limit
-in the reference's order (bit-identical), longer ones within the summation
-bound, at the row lengths and the unevenness where the rule changes."""
+in the reference's order (bit-identical), those of up to 16 entries in the
+order of a warp's tree (bit-identical), longer ones within the summation bound,
+at the row lengths and the unevenness where the rules change."""
 import numpy as np
 import pytest
 
@@ -16,12 +17,21 @@ def lengths_matrix(lengths, n_cols, seed):
     return rp, ci.astype(np.int32), rng.uniform(-1, 1, int(rp[-1]))
 
 
-# (row lengths, the limit to expect, uneven)
-CASES = {"stencil_7": ([7] * 700, 8, False), "up_to_8": ([8, 1] * 300, 8, False),
-         "up_to_9": ([9, 2] * 300, 16, False), "all_16": ([16] * 300, 16, False),
-         "up_to_17": ([17, 3] * 300, 16, False), "even_33": ([33] * 200, 16, False),
-         "one_of_33": ([33] + [4] * 900, 16, True), "one_of_32": ([32] + [3] * 900, 16, False),
-         "one_of_5000": ([5000] + [3] * 2000, 16, True)}
+def tree_sum(products):
+    """A warp's xor tree over up to 32 products: l and l + 16, then l + 8, ..."""
+    s = np.zeros(32, products.dtype)
+    s[:len(products)] += products
+    for o in (16, 8, 4, 2, 1):
+        s = s[:o] + s[o:2 * o]
+    return s[0]
+
+
+# (row lengths, uneven)
+CASES = {"stencil_7": ([7] * 700, False), "up_to_8": ([8, 1] * 300, False),
+         "up_to_9": ([9, 2] * 300, False), "all_16": ([16] * 300, False),
+         "0_to_17": (list(range(18)) * 30, False), "even_33": ([33] * 200, False),
+         "one_of_33": ([33] + [4] * 900, True), "one_of_32": ([32] + [3] * 900, False),
+         "one_of_5000": ([5000] + [3] * 2000, True)}
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
@@ -29,14 +39,14 @@ CASES = {"stencil_7": ([7] * 700, 8, False), "up_to_8": ([8, 1] * 300, 8, False)
 def test_defaults(handle, restatement, name, dtype):
     import torch
     from monolish_b200.device import Crs
-    lengths, limit, uneven = CASES[name]
+    lengths, uneven = CASES[name]
     n_cols = 6000
     rp, ci, v = lengths_matrix(lengths, n_cols, 4)
     v = v.astype(dtype)
     n = len(lengths)
     A = Crs(handle, n, n_cols, rp, ci, v)
     variant, short = A.tuning()
-    assert short == limit
+    assert short == 8
     assert variant == (0 if uneven and dtype == np.float64 else 2)
     x = W.uniform_mt(n_cols, -1, 1, 2, dtype)
     y = torch.full((n,), float("nan"), device="cuda",
@@ -44,7 +54,10 @@ def test_defaults(handle, restatement, name, dtype):
     A.matvec(torch.from_numpy(x).cuda(), y)
     got, want = y.cpu().numpy(), restatement.spmv(rp, ci, v, x)
     lens = np.diff(rp)
-    assert np.array_equal(got[lens <= limit], want[lens <= limit])
+    assert np.array_equal(got[lens <= 8], want[lens <= 8])
+    for i in np.nonzero((lens > 8) & (lens <= 32))[0]:
+        e = slice(rp[i], rp[i + 1])
+        assert got[i] == tree_sum(v[e] * x[ci[e]])
     scale = restatement.spmv(rp, ci, np.abs(v), np.abs(x))
     eps = np.finfo(dtype).eps
     assert np.all(np.abs(got - want) <= 4 * lens * eps * scale)
