@@ -531,13 +531,12 @@ int mlsh_csr_plan_create(mlsh_handle hs, int n_rows, int n_cols, int nnz,
     spmv_grids<double>(p.n_tiles, h.num_sms, p.spmv_grid);
   else
     spmv_grids<float>(p.n_tiles, h.num_sms, p.spmv_grid);
-  // What the autotuner finds is the better start until it runs.  FP64 rows far
-  // longer than the mean (columns scattered over x, the gathers' latency in
-  // front) gain from 3 CTAs per SM with three stages: Zipf(2) rows, n =
-  // 4,194,304, FP64, 219 us at {2 stages, 4 CTAs}, 188 at {3, 3}.
-  const bool uneven =
-      p.longest_row > kMaxShortRow && (int64_t)p.longest_row * n_rows > (int64_t)8 * nnz;
-  p.variant = dtype == MLSH_F64 && uneven ? 0 : kDefaultSpmvVariant;
+  // One variant for all lengths of rows until the autotuner runs.  FP64, {2
+  // stages, 4 CTAs} against {3, 3}: 256^3 stencil 264 and 289 us, Zipf(2) with n =
+  // 4,194,304 165 and 168, 2,000,000 rows of 7 with 30 % of the entries in
+  // rows of 40 / 300 / 3,000 scattered ones 69 / 68 / 94 and 74 / 68 / 101;
+  // the other way round only with few such rows (2 % in rows of 300: 39 and 35).
+  p.variant = kDefaultSpmvVariant;
   *out = ps;
   return MLSH_SUCCESS;
 }

@@ -1,7 +1,7 @@
 """The SpMV variant and short-row limit a plan starts with: rows up to the limit
 in the reference's order (bit-identical), those of up to 16 entries in the
 order of a warp's tree (bit-identical), longer ones within the summation bound,
-at the row lengths and the unevenness where the rules change."""
+at the row lengths where the rules change."""
 import numpy as np
 import pytest
 
@@ -26,12 +26,11 @@ def tree_sum(products):
     return s[0]
 
 
-# (row lengths, uneven)
-CASES = {"stencil_7": ([7] * 700, False), "up_to_8": ([8, 1] * 300, False),
-         "up_to_9": ([9, 2] * 300, False), "all_16": ([16] * 300, False),
-         "0_to_17": (list(range(18)) * 30, False), "even_33": ([33] * 200, False),
-         "one_of_33": ([33] + [4] * 900, True), "one_of_32": ([32] + [3] * 900, False),
-         "one_of_5000": ([5000] + [3] * 2000, True)}
+# row lengths
+CASES = {"stencil_7": [7] * 700, "up_to_8": [8, 1] * 300, "up_to_9": [9, 2] * 300,
+         "all_16": [16] * 300, "0_to_17": list(range(18)) * 30, "even_33": [33] * 200,
+         "one_of_33": [33] + [4] * 900, "one_of_32": [32] + [3] * 900,
+         "one_of_5000": [5000] + [3] * 2000}
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
@@ -39,15 +38,13 @@ CASES = {"stencil_7": ([7] * 700, False), "up_to_8": ([8, 1] * 300, False),
 def test_defaults(handle, restatement, name, dtype):
     import torch
     from monolish_b200.device import Crs
-    lengths, uneven = CASES[name]
+    lengths = CASES[name]
     n_cols = 6000
     rp, ci, v = lengths_matrix(lengths, n_cols, 4)
     v = v.astype(dtype)
     n = len(lengths)
     A = Crs(handle, n, n_cols, rp, ci, v)
-    variant, short = A.tuning()
-    assert short == 8
-    assert variant == (0 if uneven and dtype == np.float64 else 2)
+    assert A.tuning() == (2, 8)
     x = W.uniform_mt(n_cols, -1, 1, 2, dtype)
     y = torch.full((n,), float("nan"), device="cuda",
                    dtype=torch.float64 if dtype == np.float64 else torch.float32)
