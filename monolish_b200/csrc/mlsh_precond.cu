@@ -1387,19 +1387,22 @@ void free_dag(BlockDag &d, cudaStream_t s) {
   d.d_off = d.d_ids = nullptr;
 }
 
-// Row blocks and the lower sweep's DAG.  Blocks of 32 consecutive rows put a
+// Row blocks and the DAGs of the sweeps on them (upper: only where the matrix's
+// own upper triangle is swept; an IC factor's upper sweep runs the lower DAG
+// backwards).  Blocks of 32 consecutive rows put a
 // grid line's chain of rows into few steps, but where the line length is not
 // a multiple of 32 every block holds the end of one line and the start of the
 // next, so each block waits for the one before it and the sweep is one chain
 // of n / 32 blocks.  Ending blocks also where a row does not depend on its
 // predecessor keeps lines apart.  The cut blocks are taken when they need
-// fewer steps (counted exactly from both DAGs); when there are more than
+// fewer steps, both sweeps together (counted from the DAGs; a pattern that is
+// not symmetric can gain in one sweep what it loses in the other); when there are more than
 // eight times as many of them, too few rows share a block to be worth a look.
 // IC(0)-CG on the 49^3 7-point Laplacian: 98 levels instead of 3,677, 27.4 ms
 // per solve instead of 759; SOR-CG on a 2D grid of 8,000 rows 31.7 ms instead
 // of 86.8.  Lines of 32, 64, ... rows keep the plain blocks.
 int choose_blocks(Handle &h, const CsrPlan &p, Precond &pc, const std::vector<unsigned> &links,
-                  std::vector<int> &start, BlockDag &dag) {
+                  bool upper, std::vector<int> &start, BlockDag &dag, BlockDag &up) {
   cudaStream_t s = h.stream;
   const int n = p.n_rows;
   std::vector<int> cut;
@@ -1407,25 +1410,34 @@ int choose_blocks(Handle &h, const CsrPlan &p, Precond &pc, const std::vector<un
   block_starts(links, n, true, cut);
   const bool look = cut.size() != start.size() && cut.size() - 1 <= 8 * (start.size() - 1);
   pc.nb = (unsigned)(start.size() - 1);
+  auto build = [&](const int *d_start, const int *d_of, unsigned nb, BlockDag &lo, BlockDag &hi) {
+    int r = build_dag(h, p.row_ptr, p.col_ind, pc.lo_end, pc.up_beg, d_start, d_of, nb, false,
+                      lo);
+    if (r == MLSH_SUCCESS && upper)
+      r = build_dag(h, p.row_ptr, p.col_ind, pc.lo_end, pc.up_beg, d_start, d_of, nb, true, hi);
+    return r;
+  };
+  auto steps = [&](const BlockDag &lo, const BlockDag &hi) {
+    return dag_steps(lo, h.num_sms) + (upper ? dag_steps(hi, h.num_sms) : 0.0);
+  };
   int st = upload_blocks(start, n, &pc.blk_start, &pc.block_of, s);
-  if (st == MLSH_SUCCESS)
-    st = build_dag(h, p.row_ptr, p.col_ind, pc.lo_end, pc.up_beg, pc.blk_start, pc.block_of,
-                   pc.nb, false, dag);
+  if (st == MLSH_SUCCESS) st = build(pc.blk_start, pc.block_of, pc.nb, dag, up);
   if (st != MLSH_SUCCESS || !look) return st;
   int *c_start = nullptr, *c_of = nullptr;
-  BlockDag cd;
+  BlockDag cd, cu;
   const unsigned cnb = (unsigned)(cut.size() - 1);
   st = upload_blocks(cut, n, &c_start, &c_of, s);
-  if (st == MLSH_SUCCESS)
-    st = build_dag(h, p.row_ptr, p.col_ind, pc.lo_end, pc.up_beg, c_start, c_of, cnb, false, cd);
-  if (st == MLSH_SUCCESS && dag_steps(cd, h.num_sms) < dag_steps(dag, h.num_sms)) {
+  if (st == MLSH_SUCCESS) st = build(c_start, c_of, cnb, cd, cu);
+  if (st == MLSH_SUCCESS && steps(cd, cu) < steps(dag, up)) {
     std::swap(pc.blk_start, c_start);
     std::swap(pc.block_of, c_of);
     std::swap(dag, cd);
+    std::swap(up, cu);
     start.swap(cut);
     pc.nb = cnb;
   }
   free_dag(cd, s);
+  free_dag(cu, s);
   pool_free(c_start, s);
   pool_free(c_of, s);
   return st;
@@ -1462,16 +1474,6 @@ int build_schedule(Handle &h, const std::vector<int> &start, BlockDag &dag, bool
   return MLSH_SUCCESS;
 }
 
-// The upper sweep's schedule on the blocks the lower sweep chose.
-int build_upper(Handle &h, Precond &pc, const int *rp, const int *ci, const int *lo,
-                const int *up, const std::vector<int> &start) {
-  BlockDag dag;
-  int st = build_dag(h, rp, ci, lo, up, pc.blk_start, pc.block_of, pc.nb, true, dag);
-  if (st == MLSH_SUCCESS) st = build_schedule(h, start, dag, true, pc.sbwd);
-  free_dag(dag, h.stream);
-  return st;
-}
-
 int build_impl(Handle &h, const CsrPlan &p, int kind, double omega, bool solver_scale,
                Precond &pc) {
   cudaStream_t s = h.stream;
@@ -1500,17 +1502,16 @@ int build_impl(Handle &h, const CsrPlan &p, int kind, double omega, bool solver_
   int st = split_rows(h, p.row_ptr, p.col_ind, n, pc.lo_end, pc.up_beg, &missing, &links);
   if (st != MLSH_SUCCESS) return st;
   std::vector<int> start;
-  BlockDag dag;
-  st = choose_blocks(h, p, pc, links, start, dag);
+  BlockDag dag, up;
+  const bool upper = kind != MLSH_PRECOND_IC && !solver_scale;
+  st = choose_blocks(h, p, pc, links, upper, start, dag, up);
   if (st == MLSH_SUCCESS) st = build_schedule(h, start, dag, false, pc.sfwd);
+  if (st == MLSH_SUCCESS && upper) st = build_schedule(h, start, up, true, pc.sbwd);
   free_dag(dag, s);
+  free_dag(up, s);
   if (st != MLSH_SUCCESS) return st;
   MLSH_CUDA_TRY(pool_alloc(&pc.flags, sizeof(unsigned) * (size_t)pc.nb, s));
   MLSH_CUDA_TRY(cudaMemsetAsync(pc.flags, 0, sizeof(unsigned) * (size_t)pc.nb, s));
-  if (kind != MLSH_PRECOND_IC && !solver_scale) {
-    st = build_upper(h, pc, p.row_ptr, p.col_ind, pc.lo_end, pc.up_beg, start);
-    if (st != MLSH_SUCCESS) return st;
-  }
   if (kind == MLSH_PRECOND_SOR) {
     // M = 1/(omega d) for the preconditioner; 1/((1/omega) d) for the solver
     MLSH_CUDA_TRY(pool_alloc(&pc.scale, esz * nn, s));
@@ -1568,7 +1569,10 @@ int build_impl(Handle &h, const CsrPlan &p, int kind, double omega, bool solver_
   unsigned long long missing_t = ~0ull;
   st = split_rows(h, pc.rp_t, pc.ci_t, n, pc.lo_t, pc.up_t, &missing_t, nullptr);
   if (st != MLSH_SUCCESS) return st;
-  st = build_upper(h, pc, pc.rp_t, pc.ci_t, pc.lo_t, pc.up_t, start);
+  st = build_dag(h, pc.rp_t, pc.ci_t, pc.lo_t, pc.up_t, pc.blk_start, pc.block_of, pc.nb, true,
+                 up);
+  if (st == MLSH_SUCCESS) st = build_schedule(h, start, up, true, pc.sbwd);
+  free_dag(up, s);
   if (st != MLSH_SUCCESS) return st;
   pc.fwd = Sweep{p.row_ptr,     p.col_ind,       pc.fval,        pc.lo_end, pc.up_beg,
                  nullptr,       kDiagFwd,        pc.sfwd.order,  pc.sfwd.dep_off,

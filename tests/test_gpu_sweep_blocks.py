@@ -134,3 +134,32 @@ def test_blocks_of_uneven_rows(handle, line, lines):
         assert pc.info()[2] == host_blocks(rp, ci)
         pc.close()
     A.close()
+
+
+@pytest.mark.parametrize("kind,plain", [(SOR, True), (ILU, True), (IC, False)])
+def test_blocks_weigh_both_sweeps(handle, restatement, kind, plain):
+    """Lines of 49 rows below the diagonal, row i + 2 above it: cut blocks save
+    the lower sweep 21 levels of scans and cost the upper one 18 levels of
+    chains, which weigh three times as much.  An IC factor sweeps the lower
+    triangle both ways and takes the cut blocks."""
+    from monolish_b200 import device as D
+    line, lines = 49, 40
+    n = line * lines
+    _, rp, ci, v = W.poisson2d(line, lines)
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    low = ci <= rows
+    i = np.arange(n - 2)
+    row, col = np.concatenate([rows[low], i]), np.concatenate([ci[low], i + 2])
+    val = np.concatenate([v[low], np.full(n - 2, -0.5)])
+    o = np.lexsort((col, row))
+    rp = np.searchsorted(row[o], np.arange(n + 1)).astype(np.int32)
+    ci, v = col[o].astype(np.int32), val[o]
+    A = D.Crs(handle, n, n, rp, ci, v)
+    pc = D.Precond(A, kind, omega=1.0)
+    lower, upper, blocks = pc.info()
+    if plain:
+        assert (blocks, lower, upper) == (-(-n // 32), 62, 62)
+    else:
+        assert (blocks, lower, upper) == (host_blocks(rp, ci), 41, 41)
+    pc.close()
+    A.close()
