@@ -219,8 +219,11 @@ __global__ void gather_u32(const unsigned *src, const unsigned *perm, long long 
     dst[i] = src[perm[i]];
 }
 
-// out[j] = first position whose key is >= j, for j = 0..n_out.
-__global__ void lower_bounds(const unsigned *keys, long long n, int n_out, int *out) {
+// out[j] = first position whose key is >= j, for j = 0..n_out; nothing when a
+// check before it has set *err.
+__global__ void lower_bounds(const unsigned *keys, long long n, int n_out, int *out,
+                             const int *err) {
+  if (err != nullptr && *err != 0) return;
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j <= n_out;
        j += (long long)gridDim.x * blockDim.x) {
     long long lo = 0, hi = n;
@@ -851,7 +854,8 @@ int transpose_build(Handle &h, int n_rows, int n_cols, int nnz, const int *rp, c
                                 s));
   iota_u32<<<grid_for(nnz), 256, 0, s>>>(w.v[0], nnz);
   const int r = radix_sort_pairs(w, 0, nnz, bit_length((long long)n_cols - 1));
-  lower_bounds<<<grid_for((long long)n_cols + 1), 256, 0, s>>>(w.k[r], nnz, n_cols, rp_t);
+  lower_bounds<<<grid_for((long long)n_cols + 1), 256, 0, s>>>(w.k[r], nnz, n_cols, rp_t,
+                                                               nullptr);
   if (dtype == MLSH_F64)
     transpose_fill<double><<<grid_for(nnz), 256, 0, s>>>(
         rp, n_rows, w.v[r], nnz, static_cast<const double *>(val), ci_t,
@@ -1057,13 +1061,14 @@ int mlsh_coo_to_csr(mlsh_handle hs, int n_rows, int64_t nnz, const int *d_row, i
     return MLSH_ERR_INVALID_ARG;
   cudaStream_t s = hs->h.stream;
   // the check's word and its host mirror live with the handle; the searches
-  // stay in bounds whatever the rows hold, so one wait covers both launches
+  // read the word, so one wait covers both launches and rows that fail the
+  // check leave d_row_ptr as it was
   Handle &h = hs->h;
   int *d_err = reinterpret_cast<int *>(h.scalars + 6);
   MLSH_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s));
   if (nnz > 0) rows_sorted_check<<<grid_for(nnz), 256, 0, s>>>(d_row, nnz, n_rows, d_err);
   lower_bounds<<<grid_for((long long)n_rows + 1), 256, 0, s>>>(
-      reinterpret_cast<const unsigned *>(d_row), nnz, n_rows, d_row_ptr);
+      reinterpret_cast<const unsigned *>(d_row), nnz, n_rows, d_row_ptr, d_err);
   MLSH_CUDA_TRY(cudaGetLastError());
   MLSH_CUDA_TRY(cudaMemcpyAsync(&h.host_scalars[6], d_err, sizeof(int), cudaMemcpyDeviceToHost,
                                 s));

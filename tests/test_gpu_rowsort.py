@@ -121,3 +121,16 @@ def test_two_scatters(handle, n_rows, k, order, dtype):
     assert np.array_equal(dr.cpu().numpy()[:cnt], row[o][last])
     assert np.array_equal(dc.cpu().numpy()[:cnt], col[o][last])
     assert np.array_equal(dv.cpu().numpy()[:cnt], val[o][last])
+
+
+@pytest.mark.parametrize("row", [[0, 2, 1, 3], [0, 1, 5, 5], [-1, 0, 1, 2]])
+def test_refused_rows_leave_the_output(handle, row):
+    """Rows out of order or out of range: the error, and row_ptr as it was."""
+    import torch
+    from monolish_b200 import _abi
+    from monolish_b200.device import ptr
+    d_row = _dev(np.array(row, np.int32))
+    rp = torch.full((6,), 77, dtype=torch.int32, device="cuda")
+    st = handle.lib.mlsh_coo_to_csr(handle.h, 5, 4, ptr(d_row), ptr(rp))
+    assert st == _abi.ERR_INVALID_CSR
+    assert (rp == 77).all()
