@@ -735,18 +735,20 @@ int mlsh_nrm2_device(mlsh_handle hs, int dtype, int64_t n, const void *x,
 // store is seen earlier than a copy behind it and a stream synchronization
 // return (a step of eight vector calls on 16,383 rows, three of them waited
 // for: 64.0 us instead of 89.6).  The stream is asked now and then, so an error
-// (or a stream in capture) ends the wait.
+// (or a stream in capture) ends the wait.  The number is read with acquire
+// order, so the result read after it is the one stored before it.
 static int wait_result(Handle &h, double *host_result) {
-  const volatile unsigned long long *ready =
-      reinterpret_cast<const volatile unsigned long long *>(&h.host_scalars[3]);
-  for (unsigned spin = 1; *ready != h.dots; ++spin) {
+  const unsigned long long *ready =
+      reinterpret_cast<const unsigned long long *>(&h.host_scalars[3]);
+  auto arrived = [&] { return __atomic_load_n(ready, __ATOMIC_ACQUIRE) == h.dots; };
+  for (unsigned spin = 1; !arrived(); ++spin) {
     if ((spin & 0x3fffu) != 0) continue;
     const cudaError_t e = cudaStreamQuery(h.stream);
     if (e == cudaErrorNotReady) continue;
-    if (e == cudaSuccess && *ready == h.dots) break;
+    if (e == cudaSuccess && arrived()) break;
     // finished without the store, or failed: the stream's own verdict
     MLSH_CUDA_TRY(e == cudaSuccess ? cudaStreamSynchronize(h.stream) : e);
-    if (*ready != h.dots) return MLSH_ERR_CUDA;
+    if (!arrived()) return MLSH_ERR_CUDA;
     break;
   }
   *host_result = *(const volatile double *)&h.host_scalars[2];
