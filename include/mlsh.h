@@ -439,6 +439,9 @@ int mlsh_precond_info(mlsh_precond pc, int *levels_lower, int *levels_upper,
 #define MLSH_SWEEP_CTA 1
 #define MLSH_SWEEP_RING 2
 int mlsh_precond_sweep_form(mlsh_precond pc, int *lower, int *upper);
+/* CTAs of the cluster that runs each sweep reported as MLSH_SWEEP_FLAGS; 0
+ * where the sweep runs over the GPU with per-block flags, or in another form. */
+int mlsh_precond_sweep_ctas(mlsh_precond pc, int *lower, int *upper);
 
 /* CG / BiCGSTAB preconditioned by `pc` (the reference's solvers with
  * set_create_precond / set_apply_precond bound to equation::SOR, IC or

@@ -1795,6 +1795,13 @@ int mlsh_precond_factor(mlsh_handle hs, mlsh_precond pc, void *out) {
   return MLSH_SUCCESS;
 }
 
+int mlsh_precond_sweep_ctas(mlsh_precond pc, int *lower, int *upper) {
+  if (!pc) return MLSH_ERR_INVALID_ARG;
+  if (lower) *lower = pc->p.sfwd.ctas;
+  if (upper) *upper = pc->p.sbwd.ctas;
+  return MLSH_SUCCESS;
+}
+
 int mlsh_precond_sweep_form(mlsh_precond pc, int *lower, int *upper) {
   if (!pc) return MLSH_ERR_INVALID_ARG;
   const Precond &p = pc->p;

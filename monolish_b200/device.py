@@ -437,10 +437,17 @@ class Precond:
         return int(lo.value), int(up.value), int(nb.value)
 
     def sweep_form(self):
-        """Kernel form of the (lower, upper) sweep: 0 flags across the GPU,
-        1 single CTA, 2 single CTA with the record ring; -1 none."""
+        """Kernel form of the (lower, upper) sweep: 0 flags across the GPU or
+        one cluster (see sweep_ctas), 1 single CTA, 2 single CTA with the record
+        ring; -1 none."""
         lo, up = C.c_int(), C.c_int()
         _abi.check(self.lib.mlsh_precond_sweep_form(self.pc, C.byref(lo), C.byref(up)))
+        return int(lo.value), int(up.value)
+
+    def sweep_ctas(self):
+        """CTAs of the cluster that runs the (lower, upper) sweep; 0: none does."""
+        lo, up = C.c_int(), C.c_int()
+        _abi.check(self.lib.mlsh_precond_sweep_ctas(self.pc, C.byref(lo), C.byref(up)))
         return int(lo.value), int(up.value)
 
     def factor(self):

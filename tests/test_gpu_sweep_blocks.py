@@ -4,7 +4,7 @@ Blocks end at 32 rows and, where that shortens the dependency chain, at rows
 that do not depend on their predecessor.  Lines just below, at and above a
 block's 32 rows and twice that, lines of a few rows (where the plain blocks
 stay), and a matrix with no line structure; systems in the single-CTA, the
-cluster and the flag-synchronized sweeps.  Factors bit-identical to the sequential
+cluster and the flag-synchronized sweeps, each asserted to run in its form.  Factors bit-identical to the sequential
 restatement, applies within the sweeps' bars (1e-12 FP64 / 1e-5 FP32).
 """
 import numpy as np
@@ -61,13 +61,15 @@ MATS = {"lines_31": (W.poisson2d(31, 31)[1:], 31),
         "lines_3": (W.poisson2d(3, 40)[1:], None),
         "lines_40_of_3": (W.poisson2d(40, 3)[1:], None),
         "cube_17": (W.poisson3d(17)[1:], 33),
-        "cube_33_flags": (W.poisson3d(33)[1:], 66),
-        "grid_251_flags": (W.poisson2d(251, 251)[1:], 258),
-        # four entries a row below its block (on one cluster), five (not); the
-        # solutions are past a single CTA's shared memory in both precisions
-        "four_outside": (banded(60000, [1, 300, 600, 900, 1200], 300)[:], None),
-        "five_outside": (banded(60000, [1, 300, 600, 900, 1200, 1500], 300)[:], None),
+        "cube_33": (W.poisson3d(33)[1:], 66),
+        "grid_251": (W.poisson2d(251, 251)[1:], 258),
+        # a block's first row has four entries before its block, the one in its
+        # line among them (on one cluster), or five (not); the solutions are
+        # past a single CTA's shared memory in both precisions
+        "four_outside": (banded(60000, [1, 300, 600, 900], 300)[:], None),
+        "five_outside": (banded(60000, [1, 300, 600, 900, 1200], 300)[:], None),
         "permuted": (permuted(*W.poisson2d(30, 30)[1:], 5), None)}
+ON_CLUSTER = ("cube_33", "grid_251", "four_outside")
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
@@ -84,6 +86,7 @@ def test_odd_lines(handle, restatement, name, dtype):
         pc = D.Precond(A, kind, omega=1.9)
         lower, upper, blocks = pc.info()
         assert blocks >= (n + 31) // 32
+        assert pc.sweep_ctas() == ((16, 16) if name in ON_CLUSTER else (0, 0))
         if most is not None:
             assert max(lower, upper) <= most, (lower, upper)
         want_f, _ = restatement.precond_factor(rp, ci, v, kind, omega=1.9)
@@ -161,5 +164,24 @@ def test_blocks_weigh_both_sweeps(handle, restatement, kind, plain):
         assert (blocks, lower, upper) == (-(-n // 32), 62, 62)
     else:
         assert (blocks, lower, upper) == (host_blocks(rp, ci), 41, 41)
+    pc.close()
+    A.close()
+
+
+def test_cluster_sweeps_repeat(handle):
+    """258 levels of fewer blocks than CTAs: CTAs without a block in a level
+    run ahead of the others.  300 applies give the same bits."""
+    import torch
+    from monolish_b200 import device as D
+    (rp, ci, v), _ = MATS["grid_251"]
+    n = len(rp) - 1
+    A = D.Crs(handle, n, n, rp, ci, v)
+    pc = D.Precond(A, SOR, omega=1.9)
+    assert pc.sweep_ctas() == (16, 16)
+    r = torch.from_numpy(np.random.default_rng(3).uniform(-1, 1, n)).cuda()
+    z = [torch.zeros_like(r) for _ in range(301)]
+    for out in z:
+        pc.apply(r, out)
+    assert all(torch.equal(z[0], out) for out in z)
     pc.close()
     A.close()
