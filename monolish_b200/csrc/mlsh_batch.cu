@@ -141,6 +141,10 @@ void drop_groups(Batch &B, int kind) {
 }
 
 void free_batch(Batch &B) {
+  if (B.space && B.handle) {
+    pool_free(B.space, B.handle->stream);
+    cudaStreamSynchronize(B.handle->stream);
+  }
   for (auto &gl : B.groups)
     for (auto &g : gl)
       if (g.stream) cudaStreamDestroy(g.stream);
@@ -151,7 +155,6 @@ void free_batch(Batch &B) {
   cudaFree(B.val32);
   cudaFree(B.d_row_off);
   cudaFree(B.d_longest);
-  cudaFree(B.space);
   if (B.done_event) cudaEventDestroy(B.done_event);
 }
 
@@ -316,31 +319,34 @@ int batch_run(Handle &h, Batch &B, int kind, const void *d_b, void *d_x, const d
   MLSH_CUDA_TRY(cudaMemsetAsync(B.d_queue, 0, sizeof(unsigned) * kMaxBatchGroups, h.stream));
   const int n_groups = (int)groups.size();
   // CG: a group's slices are as wide as its longest row; the groups of longer
-  // rows, whose systems do not fit the form, get 0 slots
-  size_t space = 0;
-  for (BatchGroup &g : groups) {
-    g.slots = 0;
-    if (kind == 0) {
-      int m = 0;
-      for (int i = g.first; i < g.first + g.count; ++i)
-        m = std::max(m, B.longest[(size_t)order[(size_t)i]]);
-      g.slots = cluster_cg_slots(kind, dt, g.rpc, m);
+  // rows, whose systems do not fit the form, get 0 slots.  Without memory for
+  // the slices every group runs the row loop.
+  for (bool slices : {kind == 0, false}) {
+    size_t space = 0;
+    for (BatchGroup &g : groups) {
+      g.slots = 0;
+      if (slices) {
+        int m = 0;
+        for (int i = g.first; i < g.first + g.count; ++i)
+          m = std::max(m, B.longest[(size_t)order[(size_t)i]]);
+        g.slots = cluster_cg_slots(kind, dt, g.rpc, m);
+      }
+      g.n_clusters = cluster_max_active(kind, dt, jac, g.rpc, g.csize, g.slots);
+      if (g.n_clusters < 1) return MLSH_NOT_IMPL;
+      g.n_clusters = std::min(g.n_clusters, g.count);
+      g.space_off = space;
+      space += (size_t)g.n_clusters * g.csize * cluster_cg_workspace(dt, g.rpc, g.slots);
     }
-    g.n_clusters = cluster_max_active(kind, dt, jac, g.rpc, g.csize, g.slots);
-    if (g.n_clusters < 1) return MLSH_NOT_IMPL;
-    g.n_clusters = std::min(g.n_clusters, g.count);
-    g.space_off = space;
-    space += (size_t)g.n_clusters * g.csize * cluster_cg_workspace(dt, g.rpc, g.slots);
-  }
-  if (space > B.space_bytes) {
-    cudaFree(B.space);
+    if (space <= B.space_bytes) break;
+    pool_free(B.space, h.stream);
     B.space = nullptr;
     B.space_bytes = 0;
-    if (cudaMalloc(&B.space, space) != cudaSuccess) {
-      cudaGetLastError();
-      return MLSH_ERR_OOM;
+    if (pool_alloc(&B.space, space, h.stream) == cudaSuccess) {
+      B.space_bytes = space;
+      break;
     }
-    B.space_bytes = space;
+    cudaGetLastError();
+    B.space = nullptr;
   }
   MLSH_CUDA_TRY(cudaEventRecord(B.done_event, h.stream));
   // one stream per group, ordered after the uploads on the handle's stream

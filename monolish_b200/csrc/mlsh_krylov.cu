@@ -1265,7 +1265,7 @@ int cluster_solve_one(Kind kind, Handle &h, CsrPlan &p, const void *b, void *x,
   const int rpc = grid ? grid_cg_rows(p.dtype, n, h.num_sms)
                        : cluster_rows_for(kind == kCG ? 0 : 1, p.dtype, n, opts->cluster_rows);
   if (rpc == 0) return MLSH_NOT_IMPL;
-  const int slots = cluster_cg_slots(kind == kCG ? 0 : 1, p.dtype, rpc, p.longest_row);
+  int slots = cluster_cg_slots(kind == kCG ? 0 : 1, p.dtype, rpc, p.longest_row);
   if (grid && slots == 0) return MLSH_NOT_IMPL;
   const int csize = (int)((n + rpc - 1) / rpc);
   const bool jac = opts->precond == MLSH_PRECOND_JACOBI;
@@ -1274,9 +1274,15 @@ int cluster_solve_one(Kind kind, Handle &h, CsrPlan &p, const void *b, void *x,
   // workspace: [system record][queue] and
   //   cluster: [inverse diagonal][r0][matrix slices]
   //   grid:    [sums and barriers][p][matrix slices]
+  // (no memory for the slices: the row-loop kernel, or the kernel engine)
   int st = ensure_ws(h, 512 + (grid ? grid_cg_space(p.dtype, n, rpc, slots)
                                     : 2 * vec + csize * cluster_cg_workspace(p.dtype, rpc,
                                                                              slots)));
+  if (st == MLSH_ERR_OOM && grid) return MLSH_NOT_IMPL;
+  if (st == MLSH_ERR_OOM && slots > 0) {
+    slots = 0;
+    st = ensure_ws(h, 512 + 2 * vec);
+  }
   if (st != MLSH_SUCCESS) return st;
   char *ws = static_cast<char *>(h.ws);
   ClusterSystem *d_sys = reinterpret_cast<ClusterSystem *>(ws);

@@ -1664,8 +1664,8 @@ int build_cluster_mode(Handle &h, const Precond &pc, const Sweep &sw, Schedule &
   using R = ClusterRec<T, MODE>;
   int *index = nullptr;  // [nb] and one flag
   unsigned char *rec = nullptr;
-  MLSH_CUDA_TRY(pool_alloc(&index, sizeof(int) * ((size_t)pc.nb + 1), s));
-  if (pool_alloc(&rec, (size_t)R::kBytes * pc.nb, s) != cudaSuccess) {
+  if (pool_alloc(&index, sizeof(int) * ((size_t)pc.nb + 1), s) != cudaSuccess ||
+      pool_alloc(&rec, (size_t)R::kBytes * pc.nb, s) != cudaSuccess) {
     cudaGetLastError();
     pool_free(index, s);
     return MLSH_SUCCESS;  // no room: the flag sweep stays

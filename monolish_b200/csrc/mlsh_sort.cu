@@ -724,7 +724,9 @@ int order_all(GroupScratch &w, Handle &h, long long n, int n_keys, unsigned long
 }
 
 // COO sort by grouping; *done = false when the general sort has to take it
-// (nothing has been written then).
+// (nothing has been written then): a row is too long, or there is no memory for
+// the groups (up to 68 bytes an entry, where rows outnumber entries; the general
+// sort takes 40).
 template <typename T>
 int coo_group_sort(Handle &h, int n_rows, int n_cols, long long n, int *row, int *col, T *val,
                    bool merge, long long *total, bool *done) {
@@ -732,6 +734,7 @@ int coo_group_sort(Handle &h, int n_rows, int n_cols, long long n, int *row, int
   GroupScratch w;
   const bool large = 16 * n >= kTwoScatterBytes;
   int st = w.alloc(h, n, n_rows, large);
+  if (st == MLSH_ERR_OOM) return MLSH_SUCCESS;
   if (st != MLSH_SUCCESS) return st;
   SortFlags f;
   st = count_groups(w, h, row, col, n, n_rows, n_cols, &f);
@@ -764,6 +767,7 @@ int transpose_group(Handle &h, int n_rows, int n_cols, long long nnz, const int 
   *done = false;
   GroupScratch w;
   int st = w.alloc(h, nnz, n_cols, false);
+  if (st == MLSH_ERR_OOM) return MLSH_SUCCESS;
   if (st != MLSH_SUCCESS) return st;
   SortFlags f;
   st = count_groups(w, h, ci, nullptr, nnz, n_cols, 0, &f);
