@@ -9,7 +9,7 @@
 //     CTAs directly from their shared memory (distributed shared memory).
 //   * A global sum is one CTA-wide reduction, a broadcast of the CTA's
 //     partial into every CTA's shared memory, and one barrier.cluster;
-//     afterwards every CTA adds the same partials in rank order, so all
+//     afterwards every CTA adds the same partials in the same tree, so all
 //     CTAs hold bit-identical scalars and take identical branches.
 //   * Recurrences, stopping rule and breakdown checks are those of
 //     src/equation/cg.cpp:13-86 and src/equation/bicgstab.cpp:13-135;

@@ -36,10 +36,7 @@ constexpr unsigned kWaitPolls = kDefaultWaitPolls;  // factorizations' polls per
 constexpr unsigned kFull = 0xffffffffu;
 
 // ---- explicitly rounded arithmetic
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+// (mul_rn and sub_rn: mlsh_sweep_cluster.cuh)
 __device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
 __device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ double sqrt_rn(double a) { return __dsqrt_rn(a); }
@@ -1036,7 +1033,7 @@ size_t cluster_sweep_smem(unsigned nb, int levels, int ctas) {
 }
 
 template <typename T, int MODE>
-cudaError_t cluster_sweep_config(unsigned nb, int levels, int ctas, cudaStream_t s,
+void cluster_sweep_config(unsigned nb, int levels, int ctas, cudaStream_t s,
                                  cudaLaunchConfig_t *cfg, cudaLaunchAttribute *at) {
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = dim3((unsigned)ctas);
@@ -1049,7 +1046,6 @@ cudaError_t cluster_sweep_config(unsigned nb, int levels, int ctas, cudaStream_t
   at->val.clusterDim.z = 1;
   cfg->attrs = at;
   cfg->numAttrs = 1;
-  return cudaSuccess;
 }
 
 template <typename T, int MODE>

@@ -36,12 +36,12 @@ constexpr int kClSweepWarps = kClSweepThreads / 32;
 constexpr int kClSweepMaxCtas = 16;
 constexpr size_t kClSweepSmem = 220 * 1024;  // solution and level starts
 
-// One block: [SweepBlock][values, places of the entries outside it]
-// [finishing factor][scan coefficients].  S: the scan's type.
+// One block: [values, places of the entries outside it][finishing factor]
+// [scan coefficients].  S: the scan's type.
 template <typename T, int MODE>
 struct ClusterRec {
   using S = typename std::conditional<MODE == kSorBwd, double, T>::type;
-  static constexpr int kVal = 16;
+  static constexpr int kVal = 0;
   static constexpr int kPlace = kVal + 4 * 32 * (int)sizeof(T);
   static constexpr int kFin = kPlace + 4 * 32 * 4;
   static constexpr int kBe = kFin + 32 * (int)sizeof(T);
@@ -55,13 +55,11 @@ __device__ __forceinline__ unsigned place_of(int order_index, int within, int ct
   return (unsigned)(order_index % ctas) << 24 | (unsigned)(order_index / ctas * 32 + within);
 }
 
-// explicitly rounded, as in mlsh_precond.cu
-__device__ __forceinline__ double cl_mul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float cl_mul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double cl_sub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ float cl_sub(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ double cl_div(double a, double b) { return __ddiv_rn(a, b); }
-__device__ __forceinline__ float cl_div(float a, float b) { return __fdiv_rn(a, b); }
+// explicitly rounded (mlsh_precond.cu uses them too)
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
 
 template <typename T>
 struct ClusterSweepArgs {
@@ -153,13 +151,13 @@ __device__ __forceinline__ T cluster_row_solve(const ClusterRow<T, MODE> &r, uin
     double sacc = 0.0;  // "auto tmp = 0.0", sor_kernel.hpp:61-66
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (r.place[u] != kNoPlace) sacc = __dadd_rn(sacc, (double)cl_mul(r.v[u], x[u]));
+      if (r.place[u] != kNoPlace) sacc = __dadd_rn(sacc, (double)mul_rn(r.v[u], x[u]));
     return (T)coefficient_scan<double, true>((double)r.rhs - sacc * (double)r.fin, r.be);
   } else {
     T acc = r.rhs;
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (r.place[u] != kNoPlace) acc = cl_sub(acc, cl_mul(r.v[u], x[u]));
+      if (r.place[u] != kNoPlace) acc = sub_rn(acc, mul_rn(r.v[u], x[u]));
     T al = acc;
     if constexpr (MODE == kSorFwd) al = acc * r.fin;
     if constexpr (MODE == kDiagFwd || MODE == kDiagBwd) al = acc / r.fin;
@@ -301,7 +299,6 @@ __global__ void __launch_bounds__(256)
   else be = -(a1 / fin);
   if (lane >= bk.rows) be = S(0);
   unsigned char *rec = recs + (size_t)q * R::kBytes;
-  if (lane == 0) *reinterpret_cast<SweepBlock *>(rec) = bk;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     reinterpret_cast<T *>(rec + R::kVal)[u * 32 + lane] = v[u];
