@@ -326,12 +326,14 @@ typedef struct {
    * exit()s on a CUDA error, src/internal/monolish_internal.hpp:34-43):
    * a kernel that runs past one gives up, the call returns MLSH_ERR_TIMEOUT
    * and the handle stays usable. */
-  double time_limit;   /* wall-clock budget of one solve on the CLUSTER
-                          engine (single solves and batches), checked by the
-                          kernel at every reduction; <= 0: 60 s */
+  double time_limit;   /* wall-clock budget of one solve on the CLUSTER or
+                          GRID engine (single solves and batches), checked by
+                          the kernel at every reduction; <= 0: 60 s */
   int64_t wait_polls;  /* SOR / IC / ILU solves: polls a 32-row block makes for
-                          a block it depends on before it gives up; <= 0:
-                          2^22 (a few seconds) */
+                          a block it depends on before it gives up (sweeps on
+                          a cluster: a level's polls for the level before);
+                          <= 0: 2^22 (a few seconds; on a cluster, whose polls
+                          are of shared memory, tenths of one) */
 } mlsh_solver_opts;
 
 typedef struct {
@@ -390,14 +392,15 @@ int mlsh_bicgstab_solve_mixed(mlsh_handle handle, mlsh_csr_plan plan,
  *   MLSH_PRECOND_SOR  M = 1 / (omega * diag(A)); apply z = M^{-1} r is a
  *                     forward sweep y_i = (r_i - sum_{j<i} a_ij y_j) M_i then
  *                     a backward sweep z_i = y_i - (sum_{j>i} a_ij z_j) M_i
- *                     (src/equation/kernel/sor_kernel.hpp:42-72).  The
- *                     sweeps read the plan's values at apply time.
+ *                     (src/equation/kernel/sor_kernel.hpp:42-72).
  *   MLSH_PRECOND_IC   IC(0): L with A ~ L L^T on A's lower pattern; apply
  *                     solves L y = r, L^T z = y.
  *   MLSH_PRECOND_ILU  ILU(0): A ~ L U on A's pattern, L unit lower; apply
  *                     solves L y = r, U z = y.
  * The object refers to the plan, which must outlive it; after the plan's
- * values change, create it again (the reference builds it in every solve).
+ * values change, create it again (the reference builds it in every solve):
+ * factors, multipliers and most forms of the sweeps hold the values of its
+ * creation.
  * Apply and the solves below run on the handle's stream; one object is used
  * by one stream at a time. */
 typedef struct mlsh_precond_s *mlsh_precond;
@@ -477,7 +480,8 @@ int mlsh_sor_solve(mlsh_handle handle, mlsh_csr_plan plan, const void *d_b,
  * BiCGSTAB in FP64).
  *
  * mlsh_batch_create groups the systems by the cluster size they need
- * (largest first).  mlsh_batch_solve launches one persistent cluster
+ * (largest first); CG systems whose longest row is past the kernel for short
+ * rows make groups of their own.  mlsh_batch_solve launches one persistent cluster
  * kernel per group on its own stream; each cluster takes systems from the
  * group's queue and solves them start to finish, so systems converge (and
  * retire) independently and freed SMs go to the next group. */

@@ -27,11 +27,12 @@
 //
 // us per iteration of Jacobi-CG in FP64, row loop -> slices on a cluster /
 // slices on all SMs: 16,384 rows (2D) 6.9 -> 3.0 / 6.8; 32,761 rows 13.0 ->
-// 3.9 / 7.3; 65,536 rows 24 -> 7.6 / 7.4; 102,400 rows 31 -> 16.0 / 8.1;
-// 262,144 rows (3D) kernel engine 26.5 -> all SMs 15.2; 512,000 rows 34 -> 21.8.
+// 3.9 / 7.3; 65,536 rows 24 -> 6.7 / 7.5; 102,400 rows 31 -> 16.0 / 8.1;
+// 262,144 rows (3D) kernel engine 22.2, all SMs 15.2; 512,000 rows 29.7, 20.2.
 // A cluster is bound by the latency of its two sums and one barrier
-// (about 2 us), from 4,096 rows a CTA on by the instructions of the product
-// (about 110 per warp and slice at 1.4 per cycle); all SMs by the arrival
+// (about 2 us), from 4,096 rows a CTA on by its instructions (about 182 per
+// warp, slice and iteration, 110 of them the product's, at 1.6 per cycle on an
+// SM); all SMs by the arrival
 // counter's round trips through L2 (about 6 us an iteration).
 #pragma once
 #include <type_traits>
@@ -40,7 +41,10 @@
 
 namespace mlsh {
 
-constexpr int kCgMaxRow = 16;      // longest row the slice form takes
+// Longest row the slice form takes at all; with many rows a CTA the layout
+// below has room for fewer entries: FP64 16 up to 1,024 rows a CTA, 12 at 4,096
+// and 7 at 8,192; FP32 16 up to 8,192 and 9 at 16,384.
+constexpr int kCgMaxRow = 16;
 constexpr int kCgMaxRows = 16384;  // rows per CTA (FP32; 8,192 in FP64)
 constexpr int kCgMaxSmem = 227 * 1024 - 6144;  // dynamic; the rest is static
 constexpr int kCgRing = 3;         // most ring slices per warp

@@ -1076,7 +1076,11 @@ void destroy_entry(GraphEntry &e) {
 // 22.2, on 101^3 38.3 and 36.2, on 128^3 70.6 and 67.2; BiCGSTAB on 48^3 37.2
 // and 34.5, on 101^3 84.3 and 83.3, but on 160^3 292 and 314.  A BiCGSTAB solve
 // with one and with eight: 105^3 17.9 and 18.2 ms, 112^3 22.1 and 22.9, 124^3 30.9
-// and 33.2: systems of more than 1.1 M rows keep one.
+// and 33.2: systems of more than 1.1 M rows keep one (the line is where the
+// measured sizes cross; why the larger ones lose was not found).  A solve that
+// ends within three iterations pays for the launches that return at once: CG on
+// 101^3 rows 139 us for one iteration, 115 with one in the body; from four on
+// eight are as fast or faster.
 constexpr int kBodyIters = 8;
 constexpr int64_t kBodyItersMaxBicgstab = 1100000;
 int body_iters(Kind kind, int64_t n) {
