@@ -551,7 +551,8 @@ def run_solve(args, wl, rank, world, local):
                          "unit": "GB/s", "frac": round(achieved / peak, 4),
                          "peak_kind": peak_kind, "traffic": None,
                          "note": "whole-solve algorithmic bytes (fused minimum) / solve time"},
-            "gpu_launches": args.steps * (r.iters * (3 if wl["kind"] == "cg" else 5) + 3),
+            "gpu_launches": args.steps * solve_launches(wl["kind"], n, r.iters, args.engine,
+                                                        args.precision),
         }
         if args.precision == "mixed":
             out["dtype"] = "f32 inner / f64 refinement"
@@ -611,6 +612,17 @@ def run_solve(args, wl, rank, world, local):
     return out
 
 
+def solve_launches(kind, n, iters, engine, precision):
+    """Kernels one single solve launches: one on a cluster; on the kernel engine
+    three (BiCGSTAB five) an iteration, of which plain solves have eight in a pass
+    of the graph's loop (BiCGSTAB up to 1.1 M rows), and the start."""
+    if precision != "mixed" and engine != "kernels" and \
+            n <= (131072 if kind == "cg" else 65536):
+        return 1
+    body = 8 if precision != "mixed" and (kind == "cg" or n <= 1100000) else 1
+    return -(-iters // body) * body * (3 if kind == "cg" else 5) + 3
+
+
 # ------------------------------------------------------ preconditioners
 def precond_apply_bytes(n, nnz, pc):
     """Algorithmic bytes of one apply z = M^{-1} r (both sweeps): the stored
@@ -652,9 +664,10 @@ def run_precond(args, wl, rank, world, local):
     torch.cuda.synchronize()
     setup_ms = (time.perf_counter() - t0) * 1e3
     lv_lo, lv_up, nblocks = pc.info()
-    forms = pc.sweep_form()
     form_names = {0: "sweep_kernel (flags across the GPU)", 1: "sweep_cta_kernel (one CTA)",
                   2: "sweep_ring_kernel (one CTA, record ring)", -1: "none"}
+    forms = [f"sweep_cluster_kernel (one cluster of {ctas} CTAs)" if ctas else form_names[form]
+             for form, ctas in zip(pc.sweep_form(), pc.sweep_ctas())]
     # one apply (both sweeps) on its own
     r = torch.from_numpy(b / np.linalg.norm(b)).cuda()
     z = torch.empty_like(r)
@@ -732,8 +745,7 @@ def run_precond(args, wl, rank, world, local):
             "roofline": {"bound": "latency", "achieved": round(achieved, 1), "peak": peak,
                          "unit": "GB/s", "frac": round(achieved / peak, 4),
                          "peak_kind": peak_kind, "traffic": None,
-                         "kernel": f"lower: {form_names[forms[0]]}; upper: "
-                                   f"{form_names[forms[1]]} (one apply)",
+                         "kernel": f"lower: {forms[0]}; upper: {forms[1]} (one apply)",
                          "bytes_per_apply": B_apply,
                          "us_per_level": round(apply_ms * 1e3 / max(hops, 1), 2),
                          "note": "algorithmic bytes of one apply / apply time against HBM; the "
@@ -743,7 +755,7 @@ def run_precond(args, wl, rank, world, local):
             # per iteration: CG 6 (SpMV, x/r update, 2 sweeps, z.r, p update),
             # BiCGSTAB 9 (p, 2 sweeps, SpMV, s, 2 sweeps, SpMV, x/r); set-up of a
             # solve: CG 4 (SpMV, 2 sweeps, init), BiCGSTAB 2 (SpMV, init)
-            "gpu_launches": args.steps * (res.iters * (6 if wl["solver"] == "cg" else 9) +
+            "gpu_launches": args.steps * (-(-res.iters // 8) * 8 * (6 if wl["solver"] == "cg" else 9) +
                                           (4 if wl["solver"] == "cg" else 2)),
         }
         if world == 1 and not args.no_cpu:
@@ -851,13 +863,8 @@ def run_batch(args, wl, rank, world, local):
     for _ in range(args.warmup):
         dx.zero_()
         status, iters, resid = batch_solve()
-    n_launch = B.info("mixed" if mixed else "cg")[1]  # one launch per group
-    batch_traffic = None
-    try:
-        with open(os.path.join(ROOT, "profiles", "batch_cg.traffic.json")) as f:
-            batch_traffic = json.load(f).get("dram_bytes_per_step")
-    except (OSError, ValueError):
-        pass
+    # one launch per group, and in FP64 one that looks for the longest rows
+    n_launch = B.info("mixed")[1] if mixed else B.info("cg")[1] + 1
     clocks = ClockSampler(local)
     clocks.start()
     if world > 1:
@@ -969,14 +976,11 @@ def run_batch(args, wl, rank, world, local):
                          "peak": peak, "unit": "GB/s",
                          "frac": round(bytes_all / per_step_s / 1e9 / peak, 4),
                          "peak_kind": peak_kind,
-                         "traffic": batch_traffic if (not mixed and count_total == 2048) else None,
-                         "traffic_unit": "DRAM bytes per batch solve (all its launches)",
+                         "traffic": None,
                          "note": "fused-CG algorithmic bytes summed over systems / batch time; "
                                  "the iteration vectors live in the clusters' shared memory and "
-                                 "each system's matrix stays in L2, so DRAM moves about 5 % of "
-                                 "these bytes: a throughput figure, not a fraction of HBM "
-                                 "traffic (the batch is bound by its largest systems' "
-                                 "iteration latency)"},
+                                 "the matrices there or in L2: a throughput figure, not a "
+                                 "fraction of HBM traffic"},
             "gpu_launches": args.steps * n_launch,
         }
         if loop_ms is not None:
