@@ -1324,6 +1324,9 @@ def cpu_reference_serve(reqs, seconds):
 
 
 # ---------------------------------------------------------- reference arm
+NO_REFERENCE = {"impl": "reference",
+                "unavailable": "reference CPU build (oracle/_ref) not present: no reference source "
+                               "tree to build it from"}
 ORACLE_GEN_LIB = os.path.join(ROOT, "oracle", "_build", "libmlsh_gen_oracle.so")
 
 
@@ -1340,8 +1343,7 @@ def run_reference(args, wl, rank, world):
         reqs = serve_requests(args.size or wl["count"], seed=4)
         cb = cpu_reference_serve(reqs, seconds=60.0)
         if cb is None:
-            return {"impl": "reference", "unavailable": "reference CPU build (oracle/_ref) "
-                                                        "not present"}
+            return NO_REFERENCE
         return {"metric": METRIC_SERVE, "value": cb["value"], "unit": "solves/s",
                 "n_gpus": world, "steps": 1, "warmup": 0, "ms_per_step": None,
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -1357,6 +1359,8 @@ def run_reference(args, wl, rank, world):
         count = len(systems)
         every = max(1, count // 16)
         sec, ns, kind = cpu_reference_batch(systems, bs, tol, every, threads)
+        if sec is None:
+            return NO_REFERENCE
         value = count / sec
         return {"metric": METRIC_BATCH, "value": round(value, 3), "unit": "solves/s",
                 "n_gpus": world, "steps": 1, "warmup": 0,
@@ -1411,18 +1415,16 @@ def run_reference(args, wl, rank, world):
                         "d2h_bytes_per_step": 0}}
     import oracle
     ref = oracle.reference_or_none()
-    kind = "reference" if ref is not None else "port"
+    if ref is None:
+        return NO_REFERENCE
+    kind = "reference"
     if wl["kind"] == "spmv":
         nnz = int(rp[-1])
         vsz = 8 if wl["dtype"] == "f64" else 4
         B = spmv_bytes(n, nnz, vsz)
-        if ref is not None:
-            ref.set_threads(threads)
-            ref.spmv(rp, ci, v, x, reps=max(1, args.warmup))
-            _, mean_s, _ = ref.spmv(rp, ci, v, x, reps=args.steps)
-        else:
-            threads = 1
-            mean_s, _, _ = cpu_reference_spmv(rp, ci, v, x, args.steps, 1)
+        ref.set_threads(threads)
+        ref.spmv(rp, ci, v, x, reps=max(1, args.warmup))
+        _, mean_s, _ = ref.spmv(rp, ci, v, x, reps=args.steps)
         value = B / mean_s / 1e9
         return {"metric": METRIC_SPMV, "value": round(value, 3), "unit": "GB/s", "n_gpus": world,
                 "steps": args.steps, "warmup": args.warmup,
@@ -1438,8 +1440,6 @@ def run_reference(args, wl, rank, world):
                         "d2h_bytes_per_step": 0}}
     b = host_matvec(rp, ci, v, x)
     tol = 1e-10 * float(np.linalg.norm(b))
-    if ref is None:
-        raise SystemExit("reference CPU build missing")
     ref.set_threads(threads)
     secs = []
     for _ in range(args.steps):

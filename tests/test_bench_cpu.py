@@ -51,3 +51,13 @@ def test_reference_arm_maps_no_product_library(reference, workload):
     line = [x for x in r.stdout.splitlines() if x.startswith("MAPS")][-1]
     assert "monolish_b200/lib" not in line, line
     assert "libmlsh_gen_oracle.so" in line and "libmonolish_cpu.so" in line, line
+
+
+@pytest.mark.parametrize("workload", ["spmv_poisson3d_f64", "cg_poisson2d"])
+def test_reference_arm_without_the_reference(workload):
+    """No reference build: the arm says so and times nothing in its place."""
+    import oracle
+    if oracle.reference_or_none() is not None:
+        pytest.skip("the reference build is here")
+    out = run_ref("--workload", workload, "--size", "24")
+    assert set(out) == {"impl", "unavailable"} and out["impl"] == "reference"
