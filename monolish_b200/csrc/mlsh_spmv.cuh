@@ -387,10 +387,10 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
       const int smax = TREE ? kTreeRow : a.short_max;
       if constexpr (TREE) {
         if (ct < nrows && len <= kTreeRow) {
-          // Entries in two rounds of eight gathers; rows of up to 8 need one
+          // Entries in two passes of eight gathers; rows of up to 8 need one
           // and are added in row order.  Lane l of the xor tree adds entries l
-          // and l + 8, then l + 4's sum, l + 2's, l + 1's: round 0 takes the
-          // even entries (lane 0's sum) as 0, 8, 4, 12, 2, 10, 6, 14, round 1
+          // and l + 8, then l + 4's sum, l + 2's, l + 1's: pass 0 takes the
+          // even entries (lane 0's sum) as 0, 8, 4, 12, 2, 10, 6, 14, pass 1
           // the odd ones (lane 1's).  Absent entries are zeros, as there.
           const bool tree = len > kShortRow;
           for (int r = 0; r < (tree ? 2 : 1); ++r) {
